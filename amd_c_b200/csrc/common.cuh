@@ -221,15 +221,26 @@ __device__ __forceinline__ float warp_sum_all(float v) {
   return v;
 }
 
-// q = round-half-away(v / d) exactly as the CPU quantiser's IEEE division gives it, without paying for a division
-// per element: t = v * (1/d) is within 7e-5 of the rounded quotient (|t| <= 127), so away from a rounding
-// boundary (k + 0.5) by more than 2.5e-4 both round to the same integer; only the rare element near a boundary,
-// or a block with a denormal-range scale, takes the exact division. rinv = __frcp_rn(d), once per block.
-__device__ __forceinline__ int q8_round(float v, float d, float rinv) {
-  const float t = __fmul_rn(v, rinv);
-  const float f = fabsf(t) - truncf(fabsf(t));
-  if (!(d > 1e-30f) || fabsf(f - 0.5f) < 2.5e-4f) return (int)roundf(__fdiv_rn(v, d));
-  return (int)roundf(t);
+// q = round-half-away(fl(v / d)) exactly as the CPU quantiser's IEEE division gives it, without a division per element and
+// without a branch: with r the correctly rounded 1 / d and t = fl(v r), fl(t + (v - t d) r) is the correctly rounded quotient
+// (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", 1990), provided nothing
+// underflows; blocks with a scale below 1e-25 are worked scaled by 2^100, which changes no quotient. Half away from zero is
+// the truncation of |t| + 0.5 added towards zero. A block of zeros (d = 0) gives NaN, which converts to 0. (With the division
+// and its branch inlined 32 times, a thread's quantisation of a block took some 5000 cycles of instruction fetch.)
+struct Q8Div {
+  float s, d, r;  // 1 or 2^100; d s; 1 / (d s)
+};
+__device__ __forceinline__ Q8Div q8_div(float d) {
+  Q8Div q;
+  q.s = d > 1e-25f ? 1.0f : 0x1p100f;
+  q.d = d * q.s, q.r = __frcp_rn(q.d);
+  return q;
+}
+__device__ __forceinline__ int q8_round(float v, const Q8Div &q) {
+  v = __fmul_rn(v, q.s);
+  float t = __fmul_rn(v, q.r);
+  t = __fmaf_rn(__fmaf_rn(-t, q.d, v), q.r, t);
+  return __float2int_rz(__fadd_rz(t, copysignf(0.5f, t)));
 }
 
 // Q8 of one block of 32 floats held one per lane: writes q, d, asum of block
@@ -238,8 +249,7 @@ __device__ __forceinline__ int q8_round(float v, float d, float rinv) {
 __device__ __forceinline__ void quant_block_warp(float x, uint8_t *q, uint32_t nb, uint32_t b, int lane) {
   const float amax = warp_max(fabsf(x));
   const float d = __fdiv_rn(amax, 127.0f);
-  int v = 0;
-  if (d != 0.0f) v = q8_round(x, d, __frcp_rn(d));
+  const int v = q8_round(x, q8_div(d));
   int s = v;
   for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
   ((int8_t *)q)[32u * b + lane] = (int8_t)v;

@@ -45,13 +45,13 @@ __device__ __forceinline__ void norm_quant_vec(const float4 (&x)[ITERS], const f
     amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
     amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 2));
     amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 4));
-    const float d = __fdiv_rn(amax, 127.0f), rinv = __frcp_rn(d);
+    const float d = __fdiv_rn(amax, 127.0f);
+    const Q8Div qd = q8_div(d);
     uint32_t pk = 0u;
     int sum = 0;
 #pragma unroll
     for (int c = 0; c < 4; c++) {
-      int q = 0;
-      if (d != 0.0f) q = q8_round(v[c], d, rinv);
+      const int q = q8_round(v[c], qd);
       sum += q;
       pk |= (uint32_t)(q & 255) << (8 * c);
     }

@@ -274,13 +274,13 @@ __device__ __forceinline__ void sk_stage_quant(const float *x, uint32_t nb, uint
 #pragma unroll
     for (int j = 0; j < 16; j++) amax = fmaxf(amax, fabsf(v[j]));
     amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
-    const float d = __fdiv_rn(amax, 127.0f), rinv = __frcp_rn(d);
+    const float d = __fdiv_rn(amax, 127.0f);
+    const Q8Div qd = q8_div(d);
     uint32_t pk[4] = {0u, 0u, 0u, 0u};
     int s = 0;
 #pragma unroll
     for (int j = 0; j < 16; j++) {
-      int q = 0;
-      if (d != 0.0f) q = q8_round(v[j], d, rinv);
+      const int q = q8_round(v[j], qd);
       s += q;
       pk[j >> 2] |= (uint32_t)(q & 255) << (8 * (j & 3));
     }
@@ -311,13 +311,13 @@ __device__ __forceinline__ void sk_stage_swiglu(const float *gu, uint32_t nb, ui
 #pragma unroll
     for (int j = 0; j < 16; j++) amax = fmaxf(amax, fabsf(v[j]));
     amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, 1));
-    const float d = __fdiv_rn(amax, 127.0f), rinv = __frcp_rn(d);
+    const float d = __fdiv_rn(amax, 127.0f);
+    const Q8Div qd = q8_div(d);
     uint32_t pk[4] = {0u, 0u, 0u, 0u};
     int s = 0;
 #pragma unroll
     for (int j = 0; j < 16; j++) {
-      int q = 0;
-      if (d != 0.0f) q = q8_round(v[j], d, rinv);
+      const int q = q8_round(v[j], qd);
       s += q;
       pk[j >> 2] |= (uint32_t)(q & 255) << (8 * (j & 3));
     }
