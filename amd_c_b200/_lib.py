@@ -51,6 +51,8 @@ SIGNATURES = {
     "ie_b200_attn_persistent_scratch_bytes": (_sz, [_u32, _u32, _u32]),
     "ie_b200_attn_persistent": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _u32, _u32, _u32, _int, _u32, _vp, _vp, _vp]),
     "ie_b200_attn_prefill": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _u32, _u32, _u32, _u32, _u32, _sz, _sz, _sz, _vp]),
+    "ie_b200_attn_prefill_scratch_bytes": (_sz, [_u32, _u32, _u32]),
+    "ie_b200_attn_prefill_split": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _u32, _u32, _u32, _u32, _u32, _sz, _sz, _sz, _u32, _vp, _vp, _vp]),
     "ie_b200_argmax_part_bytes": (_sz, [_u32]),
     "ie_b200_argmax": (_int, [_vp, _u32, _vp, _u32, _sz, _sz, _vp, _vp]),
     "ie_b200_topk_scratch_bytes": (_sz, [_u32, _u32, _u32]),

@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <vector>
 
+#include "attn_prefill_tc.cuh"
 #include "common.cuh"
 #include "ie_b200_engine.h"
 #include "ie_b200_tp.h"
@@ -83,6 +84,8 @@ struct ie_b200_engine {
                              // the whole vector itself, which costs more than the launch it saves (measured at 1 and 2 GPUs)
   void *topk_scratch = nullptr;  // candidates and results of ie_b200_engine_topk
   size_t topk_bytes = 0;
+  float *pf_scratch = nullptr;   // the prompt-chunk attention's partial rows
+  uint32_t run_hi = 0;           // positions that the chunk begun last reaches (0: unknown, ops enqueued by the caller)
   void *gemm_scratch = nullptr;  // expanded activations and K-split partials of the tcgen05 GEMM
   size_t gemm_scratch_bytes = 0;
   int norm_mode = 2;         // IE_B200_NORM: 2 (default) a kernel of its own, 0 "tail": in the producing GEMV's last CTA, 1 "prologue": in the consuming GEMVs
@@ -200,9 +203,9 @@ static int launch_op(ie_b200_engine *e, const ie_b200_op &o, uint32_t t0, uint32
       char *kcl = static_cast<char *>(e->kc) + e->kv_layer_bytes * o.layer, *vcl = static_cast<char *>(e->vc) + e->kv_layer_bytes * o.layer;
       // a prompt chunk on a half-precision cache: tokens share passes over the cache on the tensor cores
       if (T > 1 && !d.kv_f32 && (d.hd == 64 || d.hd == 128) && !e->no_prefill_attn)
-        return ie_b200_attn_prefill(static_cast<float *>(at(e, o.a, o.a_stride, t0)), kcl, vcl, static_cast<float *>(at(e, o.b, o.b_stride, t0)),
-                                    at(e, o.qo, o.qo_stride, t0), pos + 1 + t0, d.n_head, d.n_kv, d.hd, d.n_ctx, T, o.a_stride, o.b_stride,
-                                    o.qo_stride, st);
+        return attn_prefill_tc(static_cast<float *>(at(e, o.a, o.a_stride, t0)), kcl, vcl, static_cast<float *>(at(e, o.b, o.b_stride, t0)),
+                               at(e, o.qo, o.qo_stride, t0), pos + 1 + t0, d.n_head, d.n_kv, d.hd, d.n_ctx, T, o.a_stride, o.b_stride, o.qo_stride,
+                               e->run_hi, e->run_hi ? e->pf_scratch : nullptr, e->err, st);
       for (uint32_t s = 0; s < T; s += e->T_att) {  // bounded scratch: at most T_att tokens per launch
         const uint32_t n = T - s < e->T_att ? T - s : e->T_att;
         int r = ie_b200_attn_decode(static_cast<float *>(at(e, o.a, o.a_stride, t0 + s)), kcl, vcl, static_cast<float *>(at(e, o.b, o.b_stride, t0 + s)),
@@ -497,7 +500,7 @@ extern "C" void ie_b200_engine_destroy(ie_b200_engine *e) {
   IEB_RELEASE(cudaFree(e->rope_sin)), IEB_RELEASE(cudaFree(e->scalars));
   IEB_RELEASE(cudaFree(e->attn_part)), IEB_RELEASE(cudaFree(e->attn_count)), IEB_RELEASE(cudaFree(e->argmax_part)), IEB_RELEASE(cudaFree(e->hist));
   IEB_RELEASE(cudaFree(e->err));
-  IEB_RELEASE(cudaFree(e->gemm_scratch)), IEB_RELEASE(cudaFree(e->topk_scratch));
+  IEB_RELEASE(cudaFree(e->gemm_scratch)), IEB_RELEASE(cudaFree(e->topk_scratch)), IEB_RELEASE(cudaFree(e->pf_scratch));
   IEB_RELEASE(cudaFree(e->d_prog)), IEB_RELEASE(cudaFree(e->sk_part)), IEB_RELEASE(cudaFree(e->sk_amax)), IEB_RELEASE(cudaFree(e->sk_bar));
   IEB_RELEASE(cudaFree(e->sk_trace));
   if (e->h_scalars) IEB_RELEASE(cudaFreeHost(e->h_scalars));
@@ -997,6 +1000,8 @@ extern "C" int ie_b200_engine_enqueue_kinds(ie_b200_engine *e, uint32_t first, u
 // once per engine (the scratch), made ready BEFORE anything of the run is enqueued: both wait for the stream, and a wait in
 // the middle of a run would wait for exchange kernels whose partners on other GPUs this thread has not enqueued yet.
 static int prepare_chunks(ie_b200_engine *e, uint32_t T) {
+  if (T > 1 && !e->pf_scratch && !e->d.kv_f32 && (e->d.hd == 64 || e->d.hd == 128) && !e->no_prefill_attn)
+    IEB_CUDA(cudaMalloc(&e->pf_scratch, attn_prefill_scratch_bytes(e->d.n_head, e->d.hd, e->d.T_max)));
   if (T < 17 || e->no_gemm || e->gemm_mma) return IE_B200_OK;
   size_t need = 0;
   for (const ie_b200_op &o : e->ops) {
@@ -1025,10 +1030,12 @@ extern "C" int ie_b200_engine_run_begin(ie_b200_engine *e, const uint32_t *toks,
   cudaStream_t st = e->stream;
   if (int r = upload_input(e, toks, T, pos, st)) return r;
   const uint32_t n_ops = (uint32_t)e->ops.size(), ih = last_only ? e->i_head : n_ops;
+  e->run_hi = pos + T;
   for (uint32_t i = 0; i < ih; i++)
     if (int r = launch_op(e, e->ops[i], 0, T, st)) return r;
   for (uint32_t i = ih; i < n_ops; i++)  // the output head for the last token only
     if (int r = launch_op(e, e->ops[i], T - 1, 1, st)) return r;
+  e->run_hi = 0;
   IEB_CUDA(cudaMemcpy2DAsync(e->h_result, 8, e->arena + e->d.argmax_off, e->d.argmax_stride ? e->d.argmax_stride : 8, 8, T, cudaMemcpyDeviceToHost, st));
   IEB_CUDA(cudaMemcpyAsync(e->h_result + 2 * e->d.T_max, e->err, 4, cudaMemcpyDeviceToHost, st));
   e->run_T = T;

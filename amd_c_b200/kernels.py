@@ -257,6 +257,21 @@ def attn_prefill(q: torch.Tensor, kc: torch.Tensor, vc: torch.Tensor, pos: torch
     return out, oq
 
 
+def attn_prefill_split(q: torch.Tensor, kc: torch.Tensor, vc: torch.Tensor, pos: torch.Tensor, n_head: int, n_kv: int, hd: int, positions: int):
+    """attn_prefill with the positions (`positions` = pos + T) split over several CTAs; returns (out, Q8 copies, error word)."""
+    lib = _lib.load()
+    T = q.shape[0]
+    out = torch.empty((T, n_head * hd), dtype=torch.float32, device=q.device)
+    nbq = n_head * hd // 32
+    oq = torch.empty((T, q8_bytes(nbq)), dtype=torch.uint8, device=q.device)
+    scratch = torch.empty(lib.ie_b200_attn_prefill_scratch_bytes(n_head, hd, T), dtype=torch.uint8, device=q.device)
+    err = torch.zeros(1, dtype=torch.int32, device=q.device)
+    check(lib.ie_b200_attn_prefill_split(q.data_ptr(), kc.data_ptr(), vc.data_ptr(), out.data_ptr(), oq.data_ptr(), pos.data_ptr(), n_head, n_kv, hd,
+                                         kc.shape[1], T, q.stride(0) * 4, n_head * hd * 4, q8_bytes(nbq), positions, scratch.data_ptr(), err.data_ptr(),
+                                         _stream()))
+    return out, oq, err
+
+
 def topk(x: torch.Tensor, K: int):
     """x: [T, n] f32 -> (values [T, K], indices [T, K] int32): per row descending, equal values by rising index."""
     x2 = x.reshape(-1, x.shape[-1])

@@ -719,6 +719,39 @@ def test_attention_prefill_chunk(ora, cuda, n_head, n_kv, hd, T, pos0):
         assert (oq[t] == ora.quant_q8(out[t])).all(), t
 
 
+@pytest.mark.parametrize("n_head,n_kv,hd,T,pos0", [(8, 2, 128, 64, 0), (8, 2, 128, 70, 58), (40, 8, 128, 256, 1000), (16, 2, 64, 130, 897), (5, 1, 128, 2, 6000),
+                                                   (3, 3, 64, 129, 127), (28, 4, 128, 37, 3)])
+@pytest.mark.parametrize("split", [False, True])
+def test_attention_prefill_tiles(cuda, n_head, n_kv, hd, T, pos0, split):
+    """The tcgen05 chunk attention at the edges of its tiles: rows that fill one or two 128-row tiles exactly or spill into the
+    next, last blocks of exactly 128 positions and ragged ones (cache rows past the last position hold NaN), one split and many.
+    Against an fp64 softmax over the same half-precision cache. Bound: q and p carry 22 bits, sums are fp32 over at most 6 002
+    terms: 2^-21 times the score's magnitude (below 32 here) per term is below 2e-5 of a term, 1e-4 of the output scale."""
+    import torch
+
+    from amd_c_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(n_head * 1000 + T)
+    n, G = pos0 + T, n_head // n_kv
+    kc, vc = (torch.randn((n_kv, n + 140, hd), generator=gen, device=cuda).half() for _ in range(2))
+    kc[:, n:], vc[:, n:] = float("nan"), float("nan")
+    q = torch.randn((T, n_head * hd), generator=gen, device=cuda)
+    pos = torch.tensor([pos0], dtype=torch.int32, device=cuda)
+    if split:
+        out, oq, err = K.attn_prefill_split(q, kc, vc, pos, n_head, n_kv, hd, n)
+        assert int(err.item()) == 0
+    else:
+        out, oq = K.attn_prefill(q, kc, vc, pos, n_head, n_kv, hd)
+    qd = q.double().view(T, n_kv, G, hd)
+    s = torch.einsum("tkgd,knd->tkgn", qd, kc[:, :n].double()) / hd ** 0.5
+    mask = torch.arange(n, device=cuda)[None, :] > (pos0 + torch.arange(T, device=cuda))[:, None]
+    p = torch.softmax(s.masked_fill(mask[:, None, None, :], float("-inf")), dim=3)
+    want = torch.einsum("tkgn,knd->tkgd", p, vc[:, :n].double()).reshape(T, n_head * hd)
+    assert torch.isfinite(out).all()
+    assert (out.double() - want).abs().max() <= 1e-4 * want.abs().max()
+    assert (oq == K.quant_q8(out)).all()
+
+
 @pytest.mark.parametrize("typ,rows,cols,T", [(synth.GGML_Q4_0, 130, 1024, 11), (synth.GGML_Q4_K, 77, 512, 16), (synth.GGML_Q6_K, 40, 18944, 5),
                                              (synth.GGML_Q4_0, 9, 64, 2), (synth.GGML_Q8_0, 130, 1024, 11), (synth.GGML_Q8_0, 40, 4096, 16)])
 def test_gemv_several_tokens_one_pass(ora, cuda, typ, rows, cols, T):
