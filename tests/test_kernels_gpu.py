@@ -771,6 +771,28 @@ def test_gemv_several_tokens_one_pass(ora, cuda, typ, rows, cols, T):
         assert (bits(y[t]) == bits(ora.gemv(kind, qw, qs, rows, cols, xq[t], res=res[t]))).all(), t
 
 
+@pytest.mark.parametrize("typ,rows,cols,T", [
+    (synth.GGML_Q4_0, 1, 64, 2), (synth.GGML_Q4_0, 17, 32 * 34, 8), (synth.GGML_Q4_0, 15, 32 * 510, 9), (synth.GGML_Q8_0, 33, 32 * 6, 3),
+    (synth.GGML_Q8_0, 16, 32 * 450, 13), (synth.GGML_Q4_0, 4801, 256, 6), (synth.GGML_Q4_K, 4752, 256, 4), (synth.GGML_Q6_K, 4737, 256, 10),
+    (synth.GGML_Q4_K, 31, 18944, 8), (synth.GGML_Q6_K, 18, 18944, 16), (synth.GGML_Q4_0, 20, 1024, 19)])
+def test_gemv_tokens_edges(ora, cuda, typ, rows, cols, T):
+    """The multi-token GEMV where it can go wrong: rows off the 16-row tiles, more tiles than the grid has slots, rows of one
+    block, of blocks that are no multiple of a stage's four, of several activation phases, both token tiles ragged."""
+    from amd_c_b200 import kernels as K
+
+    rng = np.random.default_rng(rows * 5 + T)
+    raw = synth.make_gguf_bytes(typ, rng, rows, cols)
+    kind, qw, qs = ora.repack(typ, raw, rows, cols)
+    m = K.Mat.from_gguf(typ, dev(raw, cuda), rows, cols)
+    x = rng.standard_normal((T, cols)).astype(np.float32)
+    x[0, :32] = 0.0
+    bias = rng.standard_normal(rows).astype(np.float32)
+    xq = np.stack([ora.quant_q8(x[t]) for t in range(T)])
+    y = K.gemv(m, dev(xq, cuda), bias=dev(bias, cuda)).cpu().numpy()
+    for t in range(T):
+        assert (bits(y[t]) == bits(ora.gemv(kind, qw, qs, rows, cols, xq[t], bias=bias))).all(), t
+
+
 def test_allreduce_missing_rank_gives_up(cuda, lib):
     """Failure detection without a fault: a world of two ranks whose second rank never calls. The kernel's wait for
     the peer's words is bounded (2 s): it sets the device error word to 3 and returns, the context stays usable, and
