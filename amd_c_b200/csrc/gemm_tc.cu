@@ -8,16 +8,19 @@
 // whole K in tensor memory:
 //   activations  a pre-pass expands each token's Q8 row to x = d_a * q (f32) and splits it into two f16 terms
 //                x = x_hi + x_lo (22 significant bits), stored in the order the MMA wants (cost ~ T x K, once per chunk);
-//   weights      sixteen producer warps dequantise the CTA's 256 rows of the current 32-column block (d (q - 8); d sc q -
-//                dmin mn; d sc (q - 32)) to f32 and split them the same way, w = w_hi + w_lo, straight into shared
-//                memory in the canonical K-major core-matrix layout (cost ~ rows x K, once per 256 tokens);
+//   weights      sixteen producer warps bring raw rows by cp.async (64 bytes of a row per request, four blocks at a time, the next
+//                four on their way: one row per lane touched 32 lines with every load) and turn 256 rows of the current 32-column
+//                block into two f16 terms w = w_hi + w_lo in pairs (tc_convert), straight into shared memory in the canonical
+//                K-major core-matrix layout (cost ~ rows x K, once per 256 tokens);
 //   MMA          one thread issues, per 16 columns, w_hi x_hi + w_hi x_lo + w_lo x_hi (the dropped w_lo x_lo term is
 //                below 2^-22 of a product) as tcgen05.mma kind::f16, M = 128, N = up to 256 tokens, two 128-row tiles per
-//                CTA, accumulators in tensor memory (2 x 256 columns);
-//   epilogue     the producer warps read the accumulators back (tcgen05.ld, one row and 128 tokens per thread), add bias / residual
-//                and store token rows (32 consecutive rows per warp store: coalesced).
-// A three-stage ring (64 KB per stage: 32 KB of weights, 32 KB of activations brought by one bulk copy) is handed over
-// through mbarriers; tcgen05.commit frees a stage when the MMAs that read it have completed. Matrices with few rows
+//                CTA, accumulators in tensor memory (2 x 256 columns). Up to 128 tokens, x_hi and x_lo lie side by side as one
+//                operand of twice the width and go into two accumulators: two products of w per 16 columns instead of three;
+//   epilogue     the producer warps read the accumulators back (tcgen05.ld, one row and 32 tokens per thread at a time), add bias /
+//                residual and store token rows (32 consecutive rows per warp store: coalesced).
+// Two rings, handed over with mbarriers (full: sixteen producer warps / the bulk copy's bytes; empty: tcgen05.commit): 32 KB of
+// weights and the tokens' 128 bytes each of activations per 32-column stage, as many stages as fit.
+// Matrices with few rows
 // (3584 x 18944: 14 CTAs) are split along K over grid.z, every split writing its partial sums to scratch, which a second
 // kernel adds in split order (deterministic). Every mbarrier wait is bounded by wall time and reports through the device
 // error word; tensor memory is freed on every path.
@@ -27,30 +30,42 @@
 // its largest weight (ie_b200_mat_tc_exp), each token by 2^S_n chosen from its largest Q8 scale; the epilogue multiplies row n
 // of the result by 2^-(S_w + S_n).
 //
+// Measured, before -> now: 28672 x 4096 Q4_0 77 tokens 134 -> 125 us, 128 tokens 146 -> 126, 256 tokens 166 -> 158; 3584 x 18944
+// Q6_K 77 tokens 129 -> 78, 256 tokens 151 -> 114; 37888 x 3584 Q4_K 256 tokens 154 -> 154 (17 tokens 108 -> 120: there the
+// producers wait for the first raw stage). The error against 64 bits is that of the fp32 accumulation, as before.
 // Result: equal to the one-token GEMV (which is bit-exact with the CPU) to fp32 rounding: not bit for bit, as the
 // reference's GEMM against its GEMV.
 #include <cuda_fp16.h>
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
+
 #include "common.cuh"
+#include "row_stage.cuh"
 #include "tc_common.cuh"
 
 namespace ieb {
 
-constexpr int TC_ROWS = 256, TC_TOK = 256, TC_KS = 32, TC_STAGES = 3, TC_PROD_WARPS = 16, TC_THREADS = (TC_PROD_WARPS + 2) * 32;
+constexpr int TC_ROWS = 256, TC_TOK = 256, TC_KS = 32, TC_PROD_WARPS = 16, TC_THREADS = (TC_PROD_WARPS + 2) * 32;
 constexpr int TC_A_TILE = 128 * TC_KS * 2;       // one 128-row tile, one f16 term, one stage: 8 KB
 constexpr int TC_A_STAGE = 4 * TC_A_TILE;        // two tiles x (hi, lo)
-constexpr int TC_B_TERM = TC_TOK * TC_KS * 2;    // 16 KB
-constexpr int TC_B_STAGE = 2 * TC_B_TERM;        // (hi, lo): what the pre-pass writes per (token tile, block), one bulk copy
-constexpr int TC_SMEM = TC_STAGES * (TC_A_STAGE + TC_B_STAGE) + 256;
+constexpr int TC_TOK_STAGE = 2 * TC_KS * 2;      // one token's two f16 terms of a stage: 128 B
+constexpr int TC_MAX_ST = 4;                     // stages of a ring, at most
+constexpr uint32_t TC_SMEM = 227u * 1024u - 2048u, TC_BARS = 256u;  // (2 KB stay for the static arrays)
+// tokens of tile nt, padded to what an MMA takes
+__host__ __device__ inline uint32_t tc_pad(uint32_t T, uint32_t nt) {
+  const uint32_t n = T - nt * TC_TOK < (uint32_t)TC_TOK ? T - nt * TC_TOK : (uint32_t)TC_TOK;
+  return (n + 15u) & ~15u;
+}
 
 struct TcArgs {
   const uint8_t *w;
   size_t rowb;
   uint32_t rows, nb, T;
   uint32_t blocks_per_split;
-  const uint8_t *bp;  // expanded activations: [token tile][block][hi | lo][4 chunks][32 groups][8 tokens][8 halves]
+  const uint8_t *bp;  // expanded activations: [token tile][block][4 chunks][hi | lo][n / 8 groups][8 tokens][8 halves], n = tc_pad
+  uint32_t sa, sb;    // stages of the two rings
   float *y;
   const float *bias, *res;
   size_t ys, rs;
@@ -82,10 +97,13 @@ __global__ void __launch_bounds__(256) tc_tokscale_kernel(const uint8_t *xq, siz
 
 // ---- activations: Q8 rows -> f16 hi / lo in MMA order -----------------------------------------------------------------
 // grid (nb, token tiles), 256 threads: thread = token of the tile; writes its 32 values of the block as 4 + 4 16-byte
-// pieces (consecutive tokens write consecutive pieces). Tokens past T are zero.
+// pieces (consecutive tokens write consecutive pieces). Tokens past T are zero. The four columns of an activation word are
+// stored in the order 0, 2, 1, 3, as the producers store the weights: a mask takes bytes 0 and 2 of a word into a pair of
+// halves at once, and the order of the columns of a product does not matter.
 __global__ void __launch_bounds__(256) tc_expand_kernel(const uint8_t *xq, size_t xs, uint32_t T, uint32_t nb, const float *tok_scale, uint8_t *bp) {
   pdl_prologue();
-  const uint32_t b = blockIdx.x, nt = blockIdx.y, nl = threadIdx.x, n = nt * TC_TOK + nl;
+  const uint32_t b = blockIdx.x, nt = blockIdx.y, nl = threadIdx.x, n = nt * TC_TOK + nl, pad = tc_pad(T, nt);
+  if (nl >= pad) return;
   uint4 hi[4], lo[4];
 #pragma unroll
   for (int c = 0; c < 4; c++) hi[c] = lo[c] = make_uint4(0u, 0u, 0u, 0u);
@@ -100,116 +118,120 @@ __global__ void __launch_bounds__(256) tc_expand_kernel(const uint8_t *xq, size_
 #pragma unroll
       for (int p = 0; p < 4; p++) {
         const uint32_t wd = qw[2 * c + (p >> 1)];
-        const int s0 = (int)(int8_t)(wd >> (16 * (p & 1))), s1 = (int)(int8_t)(wd >> (16 * (p & 1) + 8));
+        const int s0 = (int)(int8_t)(wd >> (8 * (p & 1))), s1 = (int)(int8_t)(wd >> (8 * (p & 1) + 16));
         tc_split2(__fmul_rn(d, (float)s0), __fmul_rn(d, (float)s1), h[p], l[p]);
       }
       hi[c] = make_uint4(h[0], h[1], h[2], h[3]), lo[c] = make_uint4(l[0], l[1], l[2], l[3]);
     }
   }
-  uint8_t *base = bp + ((size_t)nt * nb + b) * TC_B_STAGE + (nl >> 3) * 128u + (nl & 7u) * 16u;
+  uint8_t *base = bp + (size_t)nt * nb * TC_TOK * TC_TOK_STAGE + (size_t)b * pad * TC_TOK_STAGE + nl * 16u;
 #pragma unroll
-  for (int c = 0; c < 4; c++) {
-    *reinterpret_cast<uint4 *>(base + c * 4096u) = hi[c];
-    *reinterpret_cast<uint4 *>(base + TC_B_TERM + c * 4096u) = lo[c];
+  for (uint32_t c = 0; c < 4; c++) {
+    *reinterpret_cast<uint4 *>(base + c * pad * 32u) = hi[c];
+    *reinterpret_cast<uint4 *>(base + c * pad * 32u + pad * 16u) = lo[c];
   }
 }
 
-// ---- weights: one 32-weight block of one row -> 32 floats in column order --------------------------------------------
+// ---- weights: half a block (16 columns) of one row of a raw stage -> two f16 terms, column pairs (0, 2), (1, 3) per word ----
+// Q4_0, Q8_0, Q6_K: the integer weight is exact in f16 (a byte ORed into 0x6400 is 1024 + byte), and so is the rest of a
+// product of two halves, which one fma gives: hi = rn(s q), lo = s q - hi, two weights per instruction. A Q6_K scale d sc has
+// 19 bits: s = s_hi + s_lo, lo = (s_hi q - hi) + s_lo q. Q4_K (d sc q - dmin mn cancels) is worked in f32 and split after.
+// About 2 (Q4_0) to 5 (Q4_K) instructions per weight; converting each to f32, scaling and splitting there took more than 10.
+__device__ __forceinline__ uint32_t h2u(__half2 h) { return *reinterpret_cast<const uint32_t *>(&h); }
+__device__ __forceinline__ __half2 u2h(uint32_t u) { return *reinterpret_cast<const __half2 *>(&u); }
+
 template <int KIND>
-struct TcBlk;
-template <>
-struct TcBlk<IE_B200_MAT_Q4> {
-  uint4 w;
-  uint16_t d;
-  __device__ __forceinline__ void load(const uint8_t *rp, uint32_t b, uint32_t nb) {
-    w = __ldg(reinterpret_cast<const uint4 *>(rp + 16u * (size_t)b));
-    d = __ldg(reinterpret_cast<const uint16_t *>(rp + 16u * (size_t)nb + 2u * b));
-  }
-  // columns 16 hf .. 16 hf + 15 of the block: the low (hf = 0) or high nibbles of the four words
-  __device__ __forceinline__ void values16(float (&f)[16], uint32_t, uint32_t hf) const {
-    const float df = h2f(d);
-    const uint32_t ww[4] = {w.x >> (4u * hf), w.y >> (4u * hf), w.z >> (4u * hf), w.w >> (4u * hf)};
+__device__ __forceinline__ void tc_convert(const uint8_t *raw, uint32_t r, uint32_t i, uint32_t b, uint32_t hf, float w_scale, uint32_t (&hi)[8], uint32_t (&lo)[8]) {
+  if (KIND == IE_B200_MAT_Q8) {
+    const uint4 v4 = *reinterpret_cast<const uint4 *>(raw + r * 128u + (((2u * i + hf) ^ (r & 7u)) << 4));
+    const uint32_t v[4] = {v4.x, v4.y, v4.z, v4.w};
+    const __half2 d2 = __float2half2_rn(__fmul_rn(h2f(*reinterpret_cast<const uint16_t *>(raw + 2048u + 8u * r + 2u * i)), w_scale));
+    const __half2 off = u2h(0x64806480u);  // 1152
 #pragma unroll
-    for (int j = 0; j < 16; j++) f[j] = __fmul_rn(df, (float)((int)((ww[j >> 2] >> (8 * (j & 3))) & 15u) - 8));
-  }
-};
-template <>
-struct TcBlk<IE_B200_MAT_Q8> {
-  uint4 w0, w1;
-  uint16_t d;
-  __device__ __forceinline__ void load(const uint8_t *rp, uint32_t b, uint32_t nb) {
-    w0 = __ldg(reinterpret_cast<const uint4 *>(rp + 32u * (size_t)b));
-    w1 = __ldg(reinterpret_cast<const uint4 *>(rp + 32u * (size_t)b + 16u));
-    d = __ldg(reinterpret_cast<const uint16_t *>(rp + 32u * (size_t)nb + 2u * b));
-  }
-  // columns 16 hf .. 16 hf + 15: the signed bytes of the first (hf = 0) or second four words
-  __device__ __forceinline__ void values16(float (&f)[16], uint32_t, uint32_t hf) const {
-    const float df = h2f(d);
-    const uint4 v = hf ? w1 : w0;
-    const uint32_t ww[4] = {v.x, v.y, v.z, v.w};
+    for (int k = 0; k < 4; k++) {
+      const uint32_t u = v[k] ^ 0x80808080u;  // byte + 128
 #pragma unroll
-    for (int j = 0; j < 16; j++) f[j] = __fmul_rn(df, (float)(int8_t)(ww[j >> 2] >> (8 * (j & 3))));
+      for (int p = 0; p < 2; p++) {
+        const __half2 q = __hsub2(u2h(__byte_perm(u, 0x64646464u, p ? 0x4341 : 0x4240)), off), h = __hmul2(d2, q);
+        hi[2 * k + p] = h2u(h), lo[2 * k + p] = h2u(__hfma2(d2, q, __hneg2(h)));
+      }
+    }
+    return;
   }
-};
-template <>
-struct TcBlk<IE_B200_MAT_Q4K> {
-  uint4 w, h;
-  __device__ __forceinline__ void load(const uint8_t *rp, uint32_t b, uint32_t nb) {
-    w = __ldg(reinterpret_cast<const uint4 *>(rp + 16u * (size_t)b));
-    h = __ldg(reinterpret_cast<const uint4 *>(rp + 16u * (size_t)nb + 16u * (b >> 3)));
-  }
-  __device__ __forceinline__ void values16(float (&f)[16], uint32_t b, uint32_t hf) const {
-    const uint32_t fld = q4k_field(h, (int)(b & 7u));
-    const float s = __fmul_rn(h2f((uint16_t)(h.x & 0xFFFFu)), (float)(fld & 63u));
-    const float mm = __fmul_rn(h2f((uint16_t)(h.x >> 16)), (float)(fld >> 6));
-    const uint32_t ww[4] = {w.x >> (4u * hf), w.y >> (4u * hf), w.z >> (4u * hf), w.w >> (4u * hf)};
+  const uint4 v4 = *reinterpret_cast<const uint4 *>(raw + r * 64u + ((i ^ ((r >> 1) & 3u)) << 4));
+  const uint32_t v[4] = {v4.x >> (4u * hf), v4.y >> (4u * hf), v4.z >> (4u * hf), v4.w >> (4u * hf)};
+  if (KIND == IE_B200_MAT_Q4) {
+    const __half2 d2 = __float2half2_rn(__fmul_rn(h2f(*reinterpret_cast<const uint16_t *>(raw + 1024u + 8u * r + 2u * i)), w_scale));
+    const __half2 off = u2h(0x64086408u);  // 1032
 #pragma unroll
-    for (int j = 0; j < 16; j++) f[j] = __fmaf_rn(s, (float)((ww[j >> 2] >> (8 * (j & 3))) & 15u), -mm);
-  }
-};
-template <>
-struct TcBlk<IE_B200_MAT_Q6K> {
-  uint4 w;
-  uint2 hw;
-  uint16_t sc, d;
-  __device__ __forceinline__ void load(const uint8_t *rp, uint32_t b, uint32_t nb) {
-    w = __ldg(reinterpret_cast<const uint4 *>(rp + 16u * (size_t)b));
-    hw = __ldg(reinterpret_cast<const uint2 *>(rp + 16u * (size_t)nb + 8u * b));
-    sc = __ldg(reinterpret_cast<const uint16_t *>(rp + 24u * (size_t)nb + 2u * b));
-    d = __ldg(reinterpret_cast<const uint16_t *>(rp + 26u * (size_t)nb + 2u * (b >> 3)));
-  }
-  __device__ __forceinline__ void values16(float (&f)[16], uint32_t, uint32_t hf) const {
-    const float s = __fmul_rn(h2f(d), (float)(int8_t)(hf ? sc >> 8 : sc & 255u));
-    const uint32_t ww[4] = {w.x >> (4u * hf), w.y >> (4u * hf), w.z >> (4u * hf), w.w >> (4u * hf)}, hh = hf ? hw.y : hw.x;
+    for (int k = 0; k < 4; k++) {
 #pragma unroll
-    for (int j = 0; j < 16; j++) {
-      // weight 16 hf + 4 k + i: nibble hf of byte i of word k; its two high bits at bits 8 i + 2 k of the half's high-bit word
-      const int k = j >> 2, i = j & 3;
-      const uint32_t lo4 = (ww[k] >> (8 * i)) & 15u, hi2 = (hh >> (8 * i + 2 * k)) & 3u;
-      f[j] = __fmul_rn(s, (float)((int)(lo4 | (hi2 << 4)) - 32));
+      for (int p = 0; p < 2; p++) {
+        const __half2 q = __hsub2(u2h(((v[k] >> (8 * p)) & 0x000F000Fu) | 0x64006400u), off), h = __hmul2(d2, q);
+        hi[2 * k + p] = h2u(h), lo[2 * k + p] = h2u(__hfma2(d2, q, __hneg2(h)));
+      }
+    }
+  } else if (KIND == IE_B200_MAT_Q6K) {
+    const uint32_t hw = *reinterpret_cast<const uint32_t *>(raw + 1024u + 32u * r + 8u * i + 4u * hf);
+    const uint32_t sc = raw[1536u + 8u * r + 2u * i + hf];
+    const float df = h2f(*reinterpret_cast<const uint16_t *>(raw + 1664u + 4u * r + 2u * ((b >> 3) & 1u)));
+    const float s = __fmul_rn(__fmul_rn(df, (float)(int8_t)sc), w_scale);
+    const __half sh = __float2half_rn(s);
+    const __half2 s_hi = __half2half2(sh), s_lo = __float2half2_rn(s - __half2float(sh)), off = u2h(0x64206420u);  // 1056
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint32_t w6 = (v[k] & 0x0F0F0F0Fu) | (((hw >> (2 * k)) & 0x03030303u) << 4);
+#pragma unroll
+      for (int p = 0; p < 2; p++) {
+        const __half2 q = __hsub2(u2h(((w6 >> (8 * p)) & 0x003F003Fu) | 0x64006400u), off), h = __hmul2(s_hi, q);
+        hi[2 * k + p] = h2u(h), lo[2 * k + p] = h2u(__hfma2(s_lo, q, __hfma2(s_hi, q, __hneg2(h))));
+      }
+    }
+  } else {
+    const uint4 hd = *reinterpret_cast<const uint4 *>(raw + 1024u + 16u * r);
+    const uint32_t fld = q4k_field(hd, (int)(b & 7u));
+    const float s = __fmul_rn(__fmul_rn(h2f((uint16_t)(hd.x & 0xFFFFu)), (float)(fld & 63u)), w_scale);
+    const float mm = -__fmul_rn(__fmul_rn(h2f((uint16_t)(hd.x >> 16)), (float)(fld >> 6)), w_scale);
+    const f32x2 s2 = pk2(s, s), m2 = pk2(mm, mm), two23 = pk2(-8388608.0f, -8388608.0f), neg = pk2(-1.0f, -1.0f);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint32_t u = v[k] & 0x0F0F0F0Fu;
+#pragma unroll
+      for (int p = 0; p < 2; p++) {  // a byte under 0x4B000000 is the float 2^23 + byte
+        const f32x2 q = add2(pk2(__uint_as_float(__byte_perm(u, 0x4B000000u, 0x7440 + p)), __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7442 + p))), two23);
+        const f32x2 f = fma2(s2, q, m2);
+        float f0, f1;
+        unpk2(f, f0, f1);
+        const __half2 h = __floats2half2_rn(f0, f1);
+        const float2 hf2 = __half22float2(h);
+        unpk2(fma2(pk2(hf2.x, hf2.y), neg, f), f0, f1);
+        hi[2 * k + p] = h2u(h), lo[2 * k + p] = h2u(__floats2half2_rn(f0, f1));
+      }
     }
   }
-};
+}
 
 template <int KIND>
 __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_tc[];
-  uint8_t *sA = smem_tc;                                   // [stage][tile][term] 8 KB each
-  uint8_t *sB = smem_tc + TC_STAGES * TC_A_STAGE;          // [stage][term] 16 KB each
-  uint64_t *bars = reinterpret_cast<uint64_t *>(sB + TC_STAGES * TC_B_STAGE);
-  uint64_t *full_a = bars, *full_b = bars + TC_STAGES, *empty = bars + 2 * TC_STAGES, *done = bars + 3 * TC_STAGES;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 3 * TC_STAGES + 1);
-  __shared__ uint32_t s_abort;
-  __shared__ float s_inv[TC_TOK];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t m0 = blockIdx.x * TC_ROWS, nt = blockIdx.y, split = blockIdx.z;
   const uint32_t kb0 = split * a.blocks_per_split, kb1 = min(a.nb, kb0 + a.blocks_per_split), n_it = kb1 - kb0;
-  const uint32_t n_tok = min((uint32_t)TC_TOK, a.T - nt * TC_TOK), n_eff = (n_tok + 15u) & ~15u;  // MMA N: a multiple of 16
+  const uint32_t n_eff = tc_pad(a.T, nt), b_stage = n_eff * TC_TOK_STAGE;  // MMA N: a multiple of 16
   const uint32_t n_tiles = a.rows - m0 > 128u ? 2u : 1u;
+  const bool wide = n_eff <= 128u;                         // w_hi (x_hi | x_lo) as one MMA, into two accumulators
+  uint8_t *sA = smem_tc;                                   // [stage][tile][term] 8 KB each
+  uint8_t *sB = sA + a.sa * TC_A_STAGE;                    // [stage][4 chunks][hi | lo][tokens][16 B]
+  uint8_t *sR = sB + (size_t)a.sb * min(a.T + 15u & ~15u, (uint32_t)TC_TOK) * TC_TOK_STAGE;  // raw weights: two stages per producer warp
+  uint64_t *bars = reinterpret_cast<uint64_t *>(sR + TC_PROD_WARPS * 2u * RS_BYTES<KIND>);
+  uint64_t *full_a = bars, *empty_a = bars + TC_MAX_ST, *full_b = bars + 2 * TC_MAX_ST, *empty_b = bars + 3 * TC_MAX_ST, *done = bars + 4 * TC_MAX_ST;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 4 * TC_MAX_ST + 1);
+  __shared__ uint32_t s_abort;
+  __shared__ float s_inv[TC_TOK];
 
   if (tid == 0) {
     s_abort = 0u;
-    for (int s = 0; s < TC_STAGES; s++) mbar_init(&full_a[s], (uint32_t)TC_PROD_WARPS), mbar_init(&full_b[s], 1u), mbar_init(&empty[s], 1u);
+    for (int s = 0; s < TC_MAX_ST; s++) mbar_init(&full_a[s], (uint32_t)TC_PROD_WARPS), mbar_init(&empty_a[s], 1u), mbar_init(&full_b[s], 1u), mbar_init(&empty_b[s], 1u);
     mbar_init(done, 1u);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -222,63 +244,67 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
   pdl_launch_dependents();
+  // producers: warp w dequantises 16 rows of tile w >> 3, thread = row and column half; the first raw stage (weights) is on
+  // its way before the wait for the activations
+  const uint32_t t_p = (uint32_t)warp >> 3, row0 = m0 + t_p * 128u + ((uint32_t)warp & 7u) * 16u;
+  uint8_t *raw = sR + (uint32_t)warp * 2u * RS_BYTES<KIND>;
+  if (warp < TC_PROD_WARPS) {
+    if (n_it > 0u) rs_issue<KIND>(a.w, a.rowb, a.rows, a.nb, rs_smem(raw), row0, kb0, lane);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
   pdl_wait();  // the expanded activations (and the residual) are complete
   for (uint32_t j = tid; j < TC_TOK; j += TC_THREADS) s_inv[j] = nt * TC_TOK + j < a.T ? a.tok_inv[nt * TC_TOK + j] : 0.0f;
   __syncthreads();
 
   if (warp < TC_PROD_WARPS) {
-    // ---------------- producers: warp w dequantises half h = w & 1 (16 columns) of the block for 32 rows of tile w >> 3 ----------------
-    // (16 warps of one half block per thread: four warps per scheduler hide the conversion latency behind each other; with
-    // four warps of two whole blocks per thread the tensor pipe waited for the producers)
-    const uint32_t t = (uint32_t)warp >> 3, hf = (uint32_t)warp & 1u, rl = (((uint32_t)warp >> 1) & 3u) * 32u + lane;  // tile, column half, row in the tile
-    const bool ok = m0 + t * 128u + rl < a.rows;
-    const uint8_t *rp = a.w + (size_t)(m0 + t * 128u + rl) * a.rowb;
-    TcBlk<KIND> cur, nxt, nx2;  // the blocks of this stage and of the two after it: their bytes are on the way while this one is converted
-    if (ok) {
-      if (n_it > 0u) cur.load(rp, kb0, a.nb);
-      if (n_it > 1u) nxt.load(rp, kb0 + 1u, a.nb);
-    }
+    // ---------------- producers ----------------
+    const uint32_t r = lane & 15u, hf = (uint32_t)lane >> 4, rl = ((uint32_t)warp & 7u) * 16u + r;  // row of the raw stage, column half, row in the tile
+    const uint32_t dst0 = t_p * 2 * TC_A_TILE + (rl >> 3) * 128u + (rl & 7u) * 16u + hf * 2u * 2048u;
+    uint32_t s = 0, par = 1u;  // the first round finds every stage empty
     for (uint32_t it = 0; it < n_it; it++) {
-      const uint32_t s = it % TC_STAGES, round = it / TC_STAGES, b = kb0 + it;
-      if (it + 2u < n_it && ok) nx2.load(rp, b + 2u, a.nb);
-      if (round > 0 && !mbar_wait(&empty[s], (round - 1u) & 1u, &s_abort)) break;
-      float f[16];
-      if (ok) {
-        cur.values16(f, b, hf);
-#pragma unroll
-        for (int j = 0; j < 16; j++) f[j] = __fmul_rn(f[j], a.w_scale);  // exact: a power of two
-      } else {
-#pragma unroll
-        for (int j = 0; j < 16; j++) f[j] = 0.0f;
+      const uint32_t i = it & 3u, b = kb0 + it;
+      const uint8_t *src = raw + ((it >> 2) & 1u) * RS_BYTES<KIND>;
+      if (i == 0u) {  // the next four blocks have arrived; ask for the four after them, whose place all lanes have done with
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+        if (it + 4u < n_it) rs_issue<KIND>(a.w, a.rowb, a.rows, a.nb, rs_smem(raw + (((it >> 2) + 1u) & 1u) * RS_BYTES<KIND>), row0, b + 4u, lane);
+        asm volatile("cp.async.commit_group;" ::: "memory");
       }
-      uint8_t *dst = sA + s * TC_A_STAGE + t * 2 * TC_A_TILE + (rl >> 3) * 128u + (rl & 7u) * 16u + hf * 2u * 2048u;
+      uint32_t hi[8], lo[8];
+      tc_convert<KIND>(src, r, i, b, hf, a.w_scale, hi, lo);
+      if (!mbar_wait(&empty_a[s], par, &s_abort)) break;
+      uint8_t *dst = sA + s * TC_A_STAGE + dst0;
 #pragma unroll
       for (int c = 0; c < 2; c++) {  // 8-column chunks 2 hf + c of the block
-        uint32_t h[4], l[4];
-#pragma unroll
-        for (int p = 0; p < 4; p++) tc_split2(f[8 * c + 2 * p], f[8 * c + 2 * p + 1], h[p], l[p]);
-        *reinterpret_cast<uint4 *>(dst + c * 2048u) = make_uint4(h[0], h[1], h[2], h[3]);
-        *reinterpret_cast<uint4 *>(dst + TC_A_TILE + c * 2048u) = make_uint4(l[0], l[1], l[2], l[3]);
+        *reinterpret_cast<uint4 *>(dst + c * 2048u) = make_uint4(hi[4 * c], hi[4 * c + 1], hi[4 * c + 2], hi[4 * c + 3]);
+        *reinterpret_cast<uint4 *>(dst + TC_A_TILE + c * 2048u) = make_uint4(lo[4 * c], lo[4 * c + 1], lo[4 * c + 2], lo[4 * c + 3]);
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor cores read shared memory through the async proxy
       __syncwarp();
       if (lane == 0) mbar_arrive(&full_a[s]);
-      cur = nxt, nxt = nx2;
+      if (++s == a.sa) s = 0u, par ^= 1u;
     }
     // ---------------- epilogue: accumulators -> token rows ----------------
     const bool finished = mbar_wait(done, 0u, &s_abort);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (finished && !s_abort) {
       // warp w reads lanes 32 (w & 3) .. + 31 of tensor memory (a warp reaches the quarter w mod 4 only): tile (w >> 2) & 1,
-      // token columns [128 (w >> 3), + 128)
+      // token columns 32 (w >> 3) + 64 k ..
       const uint32_t q = (uint32_t)warp & 3u, te = ((uint32_t)warp >> 2) & 1u, ch = (uint32_t)warp >> 3;
       const uint32_t row = m0 + te * 128u + q * 32u + lane;
       const float bias = (a.bias && row < a.rows && !a.partial) ? a.bias[row] : 0.0f;
       if (te < n_tiles) {
-        for (uint32_t c0 = ch * 128u; c0 < min(n_eff, ch * 128u + 128u); c0 += 32u) {
+        for (uint32_t c0 = ch * 32u; c0 < n_eff; c0 += 64u) {
           uint32_t v[32];
           tc_ld32(tmem + ((q * 32u) << 16) + te * TC_TOK + c0, v);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (wide) {
+            uint32_t v2[32];
+            tc_ld32(tmem + ((q * 32u) << 16) + te * TC_TOK + n_eff + c0, v2);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__fadd_rn(__uint_as_float(v[j]), __uint_as_float(v2[j])));
+          }
           if (row < a.rows) {
 #pragma unroll
             for (int j = 0; j < 32; j++) {
@@ -301,27 +327,32 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
   } else if (warp == TC_PROD_WARPS) {
     // ---------------- MMA issue: one thread ----------------
     if (lane == 0) {
-      // instruction descriptor: D f32, A and B f16, both K-major, N = n_eff, M = 128
-      const uint32_t idesc = (1u << 4) | ((n_eff >> 3) << 17) | ((128u >> 4) << 24);
-      bool ok = true;
-      for (uint32_t it = 0; it < n_it && ok; it++) {
-        const uint32_t s = it % TC_STAGES, par = (it / TC_STAGES) & 1u;
-        ok = mbar_wait(&full_a[s], par, &s_abort) && mbar_wait(&full_b[s], par, &s_abort);
-        if (!ok) break;
+      // instruction descriptor: D f32, A and B f16, both K-major, M = 128, N
+      const uint32_t id0 = (1u << 4) | ((128u >> 4) << 24), id_n = id0 | ((n_eff >> 3) << 17), id_2n = id0 | ((n_eff >> 2) << 17);
+      const uint32_t lbo = n_eff * 32u;  // bytes between two 8-column chunks of the activations
+      uint32_t s = 0, pa = 0, sb = 0, pb = 0;
+      for (uint32_t it = 0; it < n_it; it++) {
+        if (!mbar_wait(&full_a[s], pa, &s_abort) || !mbar_wait(&full_b[sb], pb, &s_abort)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a_base = smem_u32(sA + s * TC_A_STAGE), b_base = smem_u32(sB + s * TC_B_STAGE);
+        const uint32_t a_base = smem_u32(sA + s * TC_A_STAGE), b_base = smem_u32(sB + sb * b_stage);
         for (uint32_t t = 0; t < n_tiles; t++) {
 #pragma unroll
           for (uint32_t j = 0; j < TC_KS / 16; j++) {  // 16 columns per MMA: two 8-column core matrices
             const uint64_t a_hi = tc_desc(a_base + t * 2 * TC_A_TILE + j * 4096u, 2048u, 128u), a_lo = tc_desc(a_base + t * 2 * TC_A_TILE + TC_A_TILE + j * 4096u, 2048u, 128u);
-            const uint64_t b_hi = tc_desc(b_base + j * 8192u, 4096u, 128u), b_lo = tc_desc(b_base + TC_B_TERM + j * 8192u, 4096u, 128u);
+            const uint64_t b_hi = tc_desc(b_base + j * 2u * lbo, lbo, 128u), b_lo = tc_desc(b_base + j * 2u * lbo + n_eff * 16u, lbo, 128u);
             const uint32_t d = tmem + t * TC_TOK;
-            tc_mma(d, a_hi, b_hi, idesc, (it | j) ? 1u : 0u);
-            tc_mma(d, a_hi, b_lo, idesc, 1u);
-            tc_mma(d, a_lo, b_hi, idesc, 1u);
+            if (wide) {
+              tc_mma(d, a_hi, b_hi, id_2n, (it | j) ? 1u : 0u);
+            } else {
+              tc_mma(d, a_hi, b_hi, id_n, (it | j) ? 1u : 0u);
+              tc_mma(d, a_hi, b_lo, id_n, 1u);
+            }
+            tc_mma(d, a_lo, b_hi, id_n, 1u);
           }
         }
-        tc_commit(&empty[s]);  // arrives when the MMAs issued so far have completed: the stage may be refilled
+        tc_commit(&empty_a[s]), tc_commit(&empty_b[sb]);  // arrive when the MMAs issued so far have completed: the stages may be refilled
+        if (++s == a.sa) s = 0u, pa ^= 1u;
+        if (++sb == a.sb) sb = 0u, pb ^= 1u;
       }
       tc_commit(done);
     }
@@ -330,23 +361,24 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
     if (lane == 0) {
       uint32_t issued = 0;
       for (uint32_t it = 0; it < n_it; it++) {
-        const uint32_t s = it % TC_STAGES, round = it / TC_STAGES;
-        if (round > 0 && !mbar_wait(&empty[s], (round - 1u) & 1u, &s_abort)) break;
-        mbar_expect_tx(&full_b[s], TC_B_STAGE);
-        bulk_g2s(sB + s * TC_B_STAGE, a.bp + ((size_t)nt * a.nb + kb0 + it) * TC_B_STAGE, TC_B_STAGE, &full_b[s]);
+        const uint32_t s = it % a.sb, round = it / a.sb;
+        if (round > 0 && !mbar_wait(&empty_b[s], (round - 1u) & 1u, &s_abort)) break;
+        mbar_expect_tx(&full_b[s], b_stage);
+        bulk_g2s(sB + s * b_stage, a.bp + (size_t)nt * a.nb * TC_TOK * TC_TOK_STAGE + (size_t)(kb0 + it) * b_stage, b_stage, &full_b[s]);
         issued = it + 1u;
       }
       if (s_abort) {  // gave up: do not leave while copies are still on their way into this CTA's shared memory
-        for (uint32_t it = issued > TC_STAGES ? issued - TC_STAGES : 0u; it < issued; it++) {
+        for (uint32_t it = issued > a.sb ? issued - a.sb : 0u; it < issued; it++) {
           const uint64_t t0 = tc_now();
           uint32_t ok = 0;
           while (!ok && tc_now() - t0 < 10000000ull)
             asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-                         : "=r"(ok) : "r"(smem_u32(&full_b[it % TC_STAGES])), "r"((it / TC_STAGES) & 1u) : "memory");
+                         : "=r"(ok) : "r"(smem_u32(&full_b[it % a.sb])), "r"((it / a.sb) & 1u) : "memory");
         }
       }
     }
   }
+  if (warp < TC_PROD_WARPS) asm volatile("cp.async.wait_group 0;" ::: "memory");  // (after giving up: none is left on its way)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (tid == 0 && s_abort && a.err) atomicExch(a.err, 5u);
@@ -384,7 +416,7 @@ using namespace ieb;
 
 extern "C" size_t ie_b200_gemm_tc_scratch_bytes(uint32_t rows, uint32_t cols, uint32_t T) {
   const uint32_t nb = cols / 32u, nt = (T + TC_TOK - 1) / TC_TOK, splits = tc_splits(rows, nb, T);
-  const size_t bp = (size_t)nt * nb * TC_B_STAGE, part = splits > 1u ? (size_t)splits * T * rows * sizeof(float) : 0u;
+  const size_t bp = (size_t)nt * nb * TC_TOK * TC_TOK_STAGE, part = splits > 1u ? (size_t)splits * T * rows * sizeof(float) : 0u;
   const size_t scales = ((size_t)2 * nt * TC_TOK * sizeof(float) + 255u) & ~(size_t)255u;
   return bp + part + scales + 512u;
 }
@@ -463,7 +495,7 @@ extern "C" int ie_b200_gemm_tc(int kind, const void *d_w, uint32_t rows, uint32_
   const uint32_t nb = cols / 32u, nt = (T + TC_TOK - 1) / TC_TOK, splits = tc_splits(rows, nb, T);
   if (w_exp < -100 || w_exp > 100) return fail(IE_B200_E_ARG, "ie_b200_gemm_tc: weight exponent %d", w_exp);
   uint8_t *bp = static_cast<uint8_t *>(d_scratch);
-  const size_t bp_bytes = ((size_t)nt * nb * TC_B_STAGE + 255u) & ~(size_t)255u, sc_bytes = ((size_t)2 * nt * TC_TOK * sizeof(float) + 255u) & ~(size_t)255u;
+  const size_t bp_bytes = ((size_t)nt * nb * TC_TOK * TC_TOK_STAGE + 255u) & ~(size_t)255u, sc_bytes = ((size_t)2 * nt * TC_TOK * sizeof(float) + 255u) & ~(size_t)255u;
   float *tok_scale = reinterpret_cast<float *>(bp + bp_bytes), *tok_inv = tok_scale + (size_t)nt * TC_TOK;
   float *partial = splits > 1u ? reinterpret_cast<float *>(bp + bp_bytes + sc_bytes) : nullptr;
   IEB_LAUNCH_PDL("tc_tokscale_kernel", tc_tokscale_kernel, dim3((T + 7u) / 8u), dim3(256), 0, st, static_cast<const uint8_t *>(d_xq), x_stride, T, nb,
@@ -473,15 +505,26 @@ extern "C" int ie_b200_gemm_tc(int kind, const void *d_w, uint32_t rows, uint32_
   TcArgs a = {};
   a.w = static_cast<const uint8_t *>(d_w), a.rowb = row_bytes_of(kind, cols), a.rows = rows, a.nb = nb, a.T = T;
   a.blocks_per_split = (nb + splits - 1u) / splits;
-  if (kind != IE_B200_MAT_Q4 && kind != IE_B200_MAT_Q8) a.blocks_per_split = (a.blocks_per_split + 7u) & ~7u;
+  a.blocks_per_split = (a.blocks_per_split + 3u) & ~3u;  // whole raw stages
   a.bp = bp, a.y = d_y, a.bias = d_bias, a.res = d_res, a.ys = y_stride, a.rs = res_stride, a.partial = partial, a.err = d_err;
   a.w_scale = ldexpf(1.0f, w_exp), a.tok_inv = tok_inv;
   const uint32_t used_splits = (nb + a.blocks_per_split - 1u) / a.blocks_per_split;
   const dim3 grid((rows + TC_ROWS - 1) / TC_ROWS, nt, partial ? used_splits : 1u);
   void (*k)(TcArgs) = kind == IE_B200_MAT_Q4 ? gemm_tc_kernel<IE_B200_MAT_Q4> : kind == IE_B200_MAT_Q8 ? gemm_tc_kernel<IE_B200_MAT_Q8>
                       : kind == IE_B200_MAT_Q4K ? gemm_tc_kernel<IE_B200_MAT_Q4K> : gemm_tc_kernel<IE_B200_MAT_Q6K>;
-  if (int r = ensure_dynamic_smem(reinterpret_cast<const void *>(k), TC_SMEM)) return r;
-  IEB_LAUNCH_PDL("gemm_tc_kernel", k, grid, dim3(TC_THREADS), TC_SMEM, st, a);
+  // stages: as many as fit, the activations' ring first (its copies come from L2, the producers are next door)
+  const uint32_t bst = std::min((T + 15u) & ~15u, (uint32_t)TC_TOK) * TC_TOK_STAGE;
+  const uint32_t raw = TC_PROD_WARPS * 2u * (kind == IE_B200_MAT_Q4 ? RS_BYTES<IE_B200_MAT_Q4> : kind == IE_B200_MAT_Q8 ? RS_BYTES<IE_B200_MAT_Q8>
+                                             : kind == IE_B200_MAT_Q4K ? RS_BYTES<IE_B200_MAT_Q4K> : RS_BYTES<IE_B200_MAT_Q6K>);
+  auto smem_of = [&](uint32_t sa, uint32_t sb) { return sa * TC_A_STAGE + sb * bst + raw + TC_BARS; };
+  a.sa = a.sb = 2u;
+  for (int s = 3; s <= TC_MAX_ST; s++) {
+    if (smem_of(a.sa, a.sb + 1u) <= TC_SMEM) a.sb++;
+    if (smem_of(a.sa + 1u, a.sb) <= TC_SMEM) a.sa++;
+  }
+  const uint32_t smem = smem_of(a.sa, a.sb);
+  if (int r = ensure_dynamic_smem(reinterpret_cast<const void *>(k), smem)) return r;
+  IEB_LAUNCH_PDL("gemm_tc_kernel", k, grid, dim3(TC_THREADS), smem, st, a);
   if (partial)
     IEB_LAUNCH_PDL("tc_reduce_kernel", tc_reduce_kernel, dim3((rows + 255u) / 256u, T), dim3(256), 0, st, static_cast<const float *>(partial), used_splits, T, rows, d_y,
                    d_bias, d_res, y_stride, res_stride);
