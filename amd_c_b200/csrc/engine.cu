@@ -130,6 +130,8 @@ int ar_norm_reduce(ie_b200_allreduce *a, const float *d_part, const float *d_res
                    uint32_t n, uint32_t *d_err, cudaStream_t st, bool pushed);
 void ar_push_info(const ie_b200_allreduce *a, ArPush *out);  // allreduce.cu
 bool ar_connected(const ie_b200_allreduce *a);
+int gemm_tc_run(int kind, const void *d_w, uint32_t rows, uint32_t cols, int w_exp, const void *d_xq, float *d_y, const float *d_bias, const float *d_res, uint32_t T,
+                size_t x_stride, size_t y_stride, size_t res_stride, void *d_scratch, size_t scratch_bytes, uint32_t *d_err, cudaStream_t st, bool act_ready);  // gemm_tc.cu
 int attn_decode_fused(const float *d_q, const float *d_k, const float *d_v, void *d_kc, void *d_vc, const float *d_cos, const float *d_sin, float *d_out,
                       void *d_oq, const uint32_t *d_pos, uint32_t n_head, uint32_t n_kv, uint32_t hd, int neox, int kv_f32, uint32_t kv_len, uint32_t n_ctx,
                       void *d_part, uint32_t *d_count, cudaStream_t st, bool early);  // attn_decode.cu
@@ -138,8 +140,23 @@ int attn_decode_fused(const float *d_q, const float *d_k, const float *d_v, void
 // Can the one-token decode GEMV take this matrix?
 static bool stream_ok(const EMat &m) { return gemv_direct_ok(m.kind, m.cols); }
 
-// One op for tokens [t0, t0 + T) of a run.
-static int launch_op(ie_b200_engine *e, const ie_b200_op &o, uint32_t t0, uint32_t T, cudaStream_t st) {
+// Does the tcgen05 GEMM run op o over T tokens?
+static bool tc_gemm(const ie_b200_engine *e, const ie_b200_op &o, uint32_t T) {
+  return o.kind == IE_B200_OP_GEMV && o.mat >= 0 && (size_t)o.mat < e->mats.size() && T >= 17 && e->mats[o.mat].kind != IE_B200_MAT_F32 && !e->no_gemm &&
+         !e->gemm_mma && o.a_stride % 16u == 0;
+}
+// Are the expanded activations that GEMM op p left in the scratch also those of op o, launched right after it with nothing
+// between them (q, k and v of a layer)? The same Q8 rows, and p's result does not lie over them: all of it before or behind
+// them, or, token rows interleaved, beside them in every row.
+static bool tc_same_act(const ie_b200_engine *e, const ie_b200_op &p, const ie_b200_op &o, uint32_t T) {
+  if (!tc_gemm(e, p, T) || !tc_gemm(e, o, T) || p.a != o.a || p.a_stride != o.a_stride || e->mats[p.mat].cols != e->mats[o.mat].cols) return false;
+  const uint64_t an = e->mats[p.mat].cols / 32u * 40ull, bn = 4ull * e->mats[p.mat].rows;
+  if (p.b >= p.a + p.a_stride * (T - 1u) + an || p.a >= p.b + p.b_stride * (T - 1u) + bn) return true;
+  return p.a_stride == p.b_stride && ((p.a + an <= p.b && p.b + bn <= p.a + p.a_stride) || (p.b + bn <= p.a && p.a + an <= p.b + p.b_stride));
+}
+
+// One op for tokens [t0, t0 + T) of a run. prev: the op launched right before it for the same tokens, or NULL.
+static int launch_op(ie_b200_engine *e, const ie_b200_op &o, uint32_t t0, uint32_t T, cudaStream_t st, const ie_b200_op *prev = nullptr) {
   const ie_b200_engine_desc &d = e->d;
   void *a = at(e, o.a, o.a_stride, t0), *b = at(e, o.b, o.b_stride, t0), *c = at(e, o.c, o.c_stride, t0);
   void *qo = at(e, o.qo, o.qo_stride, t0), *res = at(e, o.res, o.res_stride, t0);
@@ -182,9 +199,10 @@ static int launch_op(ie_b200_engine *e, const ie_b200_op &o, uint32_t t0, uint32
             cudaFree(e->gemm_scratch), e->gemm_scratch = nullptr, e->gemm_scratch_bytes = 0;
             IEB_CUDA(cudaMalloc(&e->gemm_scratch, need));
             e->gemm_scratch_bytes = need;
+            prev = nullptr;
           }
-          return ie_b200_gemm_tc(mm.kind, mm.d, mm.rows, mm.cols, mm.tc_exp, a, static_cast<float *>(b), bias, static_cast<float *>(res), T, o.a_stride,
-                                 o.b_stride, o.res_stride, e->gemm_scratch, e->gemm_scratch_bytes, e->err, st);
+          return gemm_tc_run(mm.kind, mm.d, mm.rows, mm.cols, mm.tc_exp, a, static_cast<float *>(b), bias, static_cast<float *>(res), T, o.a_stride, o.b_stride,
+                             o.res_stride, e->gemm_scratch, e->gemm_scratch_bytes, e->err, st, prev && tc_same_act(e, *prev, o, T));
         }
         return ie_b200_gemm(m.kind, m.d, m.rows, m.cols, a, static_cast<float *>(b), bias, static_cast<float *>(res), T, o.a_stride, o.b_stride,
                             o.res_stride, st);
@@ -1032,7 +1050,7 @@ extern "C" int ie_b200_engine_run_begin(ie_b200_engine *e, const uint32_t *toks,
   const uint32_t n_ops = (uint32_t)e->ops.size(), ih = last_only ? e->i_head : n_ops;
   e->run_hi = pos + T;
   for (uint32_t i = 0; i < ih; i++)
-    if (int r = launch_op(e, e->ops[i], 0, T, st)) return r;
+    if (int r = launch_op(e, e->ops[i], 0, T, st, i ? &e->ops[i - 1] : nullptr)) return r;
   for (uint32_t i = ih; i < n_ops; i++)  // the output head for the last token only
     if (int r = launch_op(e, e->ops[i], T - 1, 1, st)) return r;
   e->run_hi = 0;

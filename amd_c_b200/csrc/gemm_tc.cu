@@ -12,7 +12,7 @@
 //                four on their way: one row per lane touched 32 lines with every load) and turn 256 rows of the current 32-column
 //                block into two f16 terms w = w_hi + w_lo in pairs (tc_convert), straight into shared memory in the canonical
 //                K-major core-matrix layout (cost ~ rows x K, once per 256 tokens);
-//   MMA          one thread issues, per 16 columns, w_hi x_hi + w_hi x_lo + w_lo x_hi (the dropped w_lo x_lo term is
+//   MMA          one thread per tile issues, per 16 columns, w_hi x_hi + w_hi x_lo + w_lo x_hi (the dropped w_lo x_lo term is
 //                below 2^-22 of a product) as tcgen05.mma kind::f16, M = 128, N = up to 256 tokens, two 128-row tiles per
 //                CTA, accumulators in tensor memory (2 x 256 columns). Up to 128 tokens, x_hi and x_lo lie side by side as one
 //                operand of twice the width and go into two accumulators: two products of w per 16 columns instead of three;
@@ -30,9 +30,11 @@
 // its largest weight (ie_b200_mat_tc_exp), each token by 2^S_n chosen from its largest Q8 scale; the epilogue multiplies row n
 // of the result by 2^-(S_w + S_n).
 //
-// Measured, before -> now: 28672 x 4096 Q4_0 77 tokens 134 -> 125 us, 128 tokens 146 -> 126, 256 tokens 166 -> 158; 3584 x 18944
-// Q6_K 77 tokens 129 -> 78, 256 tokens 151 -> 114; 37888 x 3584 Q4_K 256 tokens 154 -> 154 (17 tokens 108 -> 120: there the
-// producers wait for the first raw stage). The error against 64 bits is that of the fp32 accumulation, as before.
+// Measured with its pre-pass and reduction, one row per lane from global memory and every weight converted in f32 -> now: 28672 x
+// 4096 Q4_0 17 / 77 / 160 / 256 tokens 122 / 134 / 151 / 166 -> 73 / 83 / 106 / 142 us; 37888 x 3584 Q4_K 108 / 115 / 128 / 154 ->
+// 79 / 82 / 108 / 146; 3584 x 18944 Q6_K 121 / 129 / 139 / 151 -> 60 / 67 / 78 / 104. At 256 tokens the tensor pipe bounds it (three
+// products per weight and token: 126 us of f16 work for the 37888 rows at the measured bf16 burst rate).
+//
 // Result: equal to the one-token GEMV (which is bit-exact with the CPU) to fp32 rounding: not bit for bit, as the
 // reference's GEMM against its GEMV.
 #include <cuda_fp16.h>
@@ -47,7 +49,10 @@
 
 namespace ieb {
 
-constexpr int TC_ROWS = 256, TC_TOK = 256, TC_KS = 32, TC_PROD_WARPS = 16, TC_THREADS = (TC_PROD_WARPS + 2) * 32;
+int gemm_tc_run(int kind, const void *d_w, uint32_t rows, uint32_t cols, int w_exp, const void *d_xq, float *d_y, const float *d_bias, const float *d_res, uint32_t T,
+                size_t x_stride, size_t y_stride, size_t res_stride, void *d_scratch, size_t scratch_bytes, uint32_t *d_err, cudaStream_t st, bool act_ready);
+
+constexpr int TC_ROWS = 256, TC_TOK = 256, TC_KS = 32, TC_PROD_WARPS = 16, TC_THREADS = (TC_PROD_WARPS + 3) * 32;
 constexpr int TC_A_TILE = 128 * TC_KS * 2;       // one 128-row tile, one f16 term, one stage: 8 KB
 constexpr int TC_A_STAGE = 4 * TC_A_TILE;        // two tiles x (hi, lo)
 constexpr int TC_TOK_STAGE = 2 * TC_KS * 2;      // one token's two f16 terms of a stage: 128 B
@@ -72,63 +77,71 @@ struct TcArgs {
   float *partial;     // grid.z > 1: [split][T][rows]
   uint32_t *err;
   float w_scale;      // 2^S_w applied to every weight before the split
-  const float *tok_inv;  // per token: 2^-(S_w + S_n)
+  float w_inv;           // 2^-S_w
+  const float *tok_inv;  // per token: 2^-S_n
 };
 
-// One warp per token: S_n from the largest Q8 scale of the row, so that the largest |d q| 2^S_n lies in [2048, 4096];
-// tok_scale[n] = 2^S_n, tok_inv[n] = 2^-(S_n) * w_inv.
-__global__ void __launch_bounds__(256) tc_tokscale_kernel(const uint8_t *xq, size_t xs, uint32_t T, uint32_t nb, float w_inv, float *tok_scale, float *tok_inv) {
-  pdl_prologue();
-  const uint32_t n = blockIdx.x * 8u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
-  if (n >= T) return;
-  const float *d = reinterpret_cast<const float *>(xq + xs * n + 32u * (size_t)nb);
-  float m = 0.0f;
-  for (uint32_t b = lane; b < nb; b += 32u) m = fmaxf(m, fabsf(d[b]));
-  m = warp_max(m) * 127.0f;
-  int e = 0;
-  if (m > 0.0f && m < 3.0e38f) {
-    int ex;
-    frexpf(m, &ex);  // m = f * 2^ex, f in [0.5, 1)
-    e = 12 - ex;     // m * 2^e in [2048, 4096)
-    e = e > 100 ? 100 : (e < -100 ? -100 : e);
-  }
-  if (lane == 0) tok_scale[n] = ldexpf(1.0f, e), tok_inv[n] = ldexpf(w_inv, -e);
-}
-
 // ---- activations: Q8 rows -> f16 hi / lo in MMA order -----------------------------------------------------------------
-// grid (nb, token tiles), 256 threads: thread = token of the tile; writes its 32 values of the block as 4 + 4 16-byte
-// pieces (consecutive tokens write consecutive pieces). Tokens past T are zero. The four columns of an activation word are
-// stored in the order 0, 2, 1, 3, as the producers store the weights: a mask takes bytes 0 and 2 of a word into a pair of
-// halves at once, and the order of the columns of a product does not matter.
-__global__ void __launch_bounds__(256) tc_expand_kernel(const uint8_t *xq, size_t xs, uint32_t T, uint32_t nb, const float *tok_scale, uint8_t *bp) {
+// grid (groups of 8 tokens, parts of the columns), 256 threads. Warp w of a CTA first looks for the largest Q8 scale of token w
+// (every part repeats that: a few KB from L2): S_n such that the largest |d q| 2^S_n lies in [2048, 4096); tok_inv[n] = 2^-S_n.
+// Then thread = token and one of 32 blocks at a time: its 32 values as 4 + 4 16-byte pieces, eight tokens side by side. Tokens
+// past T are zero. The four columns of an activation word are stored in the order 0, 2, 1, 3, as the producers store the
+// weights: a mask takes bytes 0 and 2 of a word into a pair of halves at once, and the order of the columns of a product does
+// not matter.
+__global__ void __launch_bounds__(256) tc_expand_kernel(const uint8_t *xq, size_t xs, uint32_t T, uint32_t nb, float *tok_inv, uint8_t *bp) {
+  __shared__ float scale[8];
   pdl_prologue();
-  const uint32_t b = blockIdx.x, nt = blockIdx.y, nl = threadIdx.x, n = nt * TC_TOK + nl, pad = tc_pad(T, nt);
-  if (nl >= pad) return;
-  uint4 hi[4], lo[4];
-#pragma unroll
-  for (int c = 0; c < 4; c++) hi[c] = lo[c] = make_uint4(0u, 0u, 0u, 0u);
-  if (n < T) {
-    const uint8_t *row = xq + xs * n;
-    const uint4 q0 = *reinterpret_cast<const uint4 *>(row + 32u * b), q1 = *reinterpret_cast<const uint4 *>(row + 32u * b + 16u);
-    const float d = __fmul_rn(*reinterpret_cast<const float *>(row + 32u * (size_t)nb + 4u * b), tok_scale[n]);  // exact: a power of two
-    const uint32_t qw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-#pragma unroll
-    for (int c = 0; c < 4; c++) {  // chunk c: values 8c .. 8c + 7 = words 2c, 2c + 1
-      uint32_t h[4], l[4];
-#pragma unroll
-      for (int p = 0; p < 4; p++) {
-        const uint32_t wd = qw[2 * c + (p >> 1)];
-        const int s0 = (int)(int8_t)(wd >> (8 * (p & 1))), s1 = (int)(int8_t)(wd >> (8 * (p & 1) + 16));
-        tc_split2(__fmul_rn(d, (float)s0), __fmul_rn(d, (float)s1), h[p], l[p]);
-      }
-      hi[c] = make_uint4(h[0], h[1], h[2], h[3]), lo[c] = make_uint4(l[0], l[1], l[2], l[3]);
+  const uint32_t n0 = blockIdx.x * 8u, nt = n0 / TC_TOK, pad = tc_pad(T, nt);
+  {
+    const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31u, n = n0 + w;
+    float m = 0.0f;
+    if (n < T) {
+      const float *d = reinterpret_cast<const float *>(xq + xs * n + 32u * (size_t)nb);
+#pragma unroll 4
+      for (uint32_t b = lane; b < nb; b += 32u) m = fmaxf(m, fabsf(d[b]));
+    }
+    m = warp_max(m) * 127.0f;
+    int e = 0;
+    if (m > 0.0f && m < 3.0e38f) {
+      int ex;
+      frexpf(m, &ex);  // m = f * 2^ex, f in [0.5, 1)
+      e = 12 - ex;     // m * 2^e in [2048, 4096)
+      e = e > 100 ? 100 : (e < -100 ? -100 : e);
+    }
+    if (lane == 0) {
+      scale[w] = ldexpf(1.0f, e);
+      if (blockIdx.y == 0 && n < T) tok_inv[n] = ldexpf(1.0f, -e);
     }
   }
-  uint8_t *base = bp + (size_t)nt * nb * TC_TOK * TC_TOK_STAGE + (size_t)b * pad * TC_TOK_STAGE + nl * 16u;
+  __syncthreads();
+  const uint32_t tok = threadIdx.x & 7u, n = n0 + tok, nl = n - nt * TC_TOK;
+  for (uint32_t b = blockIdx.y * 32u + (threadIdx.x >> 3); b < nb; b += gridDim.y * 32u) {
+    uint4 hi[4], lo[4];
 #pragma unroll
-  for (uint32_t c = 0; c < 4; c++) {
-    *reinterpret_cast<uint4 *>(base + c * pad * 32u) = hi[c];
-    *reinterpret_cast<uint4 *>(base + c * pad * 32u + pad * 16u) = lo[c];
+    for (int c = 0; c < 4; c++) hi[c] = lo[c] = make_uint4(0u, 0u, 0u, 0u);
+    if (n < T) {
+      const uint8_t *row = xq + xs * n;
+      const uint4 q0 = *reinterpret_cast<const uint4 *>(row + 32u * (size_t)b), q1 = *reinterpret_cast<const uint4 *>(row + 32u * (size_t)b + 16u);
+      const float d = __fmul_rn(*reinterpret_cast<const float *>(row + 32u * (size_t)nb + 4u * b), scale[tok]);  // exact: a power of two
+      const uint32_t qw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+#pragma unroll
+      for (int c = 0; c < 4; c++) {  // chunk c: values 8c .. 8c + 7 = words 2c, 2c + 1
+        uint32_t h[4], l[4];
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+          const uint32_t wd = qw[2 * c + (p >> 1)];
+          const int s0 = (int)(int8_t)(wd >> (8 * (p & 1))), s1 = (int)(int8_t)(wd >> (8 * (p & 1) + 16));
+          tc_split2(__fmul_rn(d, (float)s0), __fmul_rn(d, (float)s1), h[p], l[p]);
+        }
+        hi[c] = make_uint4(h[0], h[1], h[2], h[3]), lo[c] = make_uint4(l[0], l[1], l[2], l[3]);
+      }
+    }
+    uint8_t *base = bp + (size_t)nt * nb * TC_TOK * TC_TOK_STAGE + (size_t)b * pad * TC_TOK_STAGE + nl * 16u;
+#pragma unroll
+    for (uint32_t c = 0; c < 4; c++) {
+      *reinterpret_cast<uint4 *>(base + c * pad * 32u) = hi[c];
+      *reinterpret_cast<uint4 *>(base + c * pad * 32u + pad * 16u) = lo[c];
+    }
   }
 }
 
@@ -231,8 +244,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
 
   if (tid == 0) {
     s_abort = 0u;
-    for (int s = 0; s < TC_MAX_ST; s++) mbar_init(&full_a[s], (uint32_t)TC_PROD_WARPS), mbar_init(&empty_a[s], 1u), mbar_init(&full_b[s], 1u), mbar_init(&empty_b[s], 1u);
-    mbar_init(done, 1u);
+    for (int s = 0; s < TC_MAX_ST; s++) mbar_init(&full_a[s], (uint32_t)TC_PROD_WARPS), mbar_init(&empty_a[s], n_tiles), mbar_init(&full_b[s], 1u), mbar_init(&empty_b[s], n_tiles);
+    mbar_init(done, n_tiles);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == TC_PROD_WARPS) {  // tensor memory: all 512 columns (two accumulators of up to 256 columns), by one warp
@@ -253,7 +266,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   pdl_wait();  // the expanded activations (and the residual) are complete
-  for (uint32_t j = tid; j < TC_TOK; j += TC_THREADS) s_inv[j] = nt * TC_TOK + j < a.T ? a.tok_inv[nt * TC_TOK + j] : 0.0f;
+  for (uint32_t j = tid; j < TC_TOK; j += TC_THREADS) s_inv[j] = nt * TC_TOK + j < a.T ? __fmul_rn(a.tok_inv[nt * TC_TOK + j], a.w_inv) : 0.0f;
   __syncthreads();
 
   if (warp < TC_PROD_WARPS) {
@@ -324,31 +337,33 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
         }
       }
     }
-  } else if (warp == TC_PROD_WARPS) {
-    // ---------------- MMA issue: one thread ----------------
-    if (lane == 0) {
+  } else if (warp < TC_PROD_WARPS + 2) {
+    // ---------------- MMA issue: one thread per tile ----------------
+    // (issuing a stage's products takes one thread longer than the tensor cores need for few tokens: 28672 x 4096, 77 tokens: 125 us
+    // with descriptors built for every product, 93 with them stepped by additions, 83 with a thread per tile)
+    const uint32_t t = (uint32_t)warp - TC_PROD_WARPS;
+    if (lane == 0 && t < n_tiles) {
       // instruction descriptor: D f32, A and B f16, both K-major, M = 128, N
       const uint32_t id0 = (1u << 4) | ((128u >> 4) << 24), id_n = id0 | ((n_eff >> 3) << 17), id_2n = id0 | ((n_eff >> 2) << 17);
       const uint32_t lbo = n_eff * 32u;  // bytes between two 8-column chunks of the activations
+      // descriptors: address fields count 16-byte units and never carry out of their 14 bits (shared memory ends at 256 KB), so
+      // a stage, a term or a column step is one addition
+      const uint64_t da0 = tc_desc(smem_u32(sA) + t * 2u * TC_A_TILE, 2048u, 128u), db0 = tc_desc(smem_u32(sB), lbo, 128u);
+      constexpr uint64_t A_LO = TC_A_TILE >> 4, A_J = 4096 >> 4;
+      const uint32_t d = tmem + t * TC_TOK;
+      const uint64_t b_j = lbo >> 3, b_lo = n_eff;
       uint32_t s = 0, pa = 0, sb = 0, pb = 0;
       for (uint32_t it = 0; it < n_it; it++) {
         if (!mbar_wait(&full_a[s], pa, &s_abort) || !mbar_wait(&full_b[sb], pb, &s_abort)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a_base = smem_u32(sA + s * TC_A_STAGE), b_base = smem_u32(sB + sb * b_stage);
-        for (uint32_t t = 0; t < n_tiles; t++) {
-#pragma unroll
-          for (uint32_t j = 0; j < TC_KS / 16; j++) {  // 16 columns per MMA: two 8-column core matrices
-            const uint64_t a_hi = tc_desc(a_base + t * 2 * TC_A_TILE + j * 4096u, 2048u, 128u), a_lo = tc_desc(a_base + t * 2 * TC_A_TILE + TC_A_TILE + j * 4096u, 2048u, 128u);
-            const uint64_t b_hi = tc_desc(b_base + j * 2u * lbo, lbo, 128u), b_lo = tc_desc(b_base + j * 2u * lbo + n_eff * 16u, lbo, 128u);
-            const uint32_t d = tmem + t * TC_TOK;
-            if (wide) {
-              tc_mma(d, a_hi, b_hi, id_2n, (it | j) ? 1u : 0u);
-            } else {
-              tc_mma(d, a_hi, b_hi, id_n, (it | j) ? 1u : 0u);
-              tc_mma(d, a_hi, b_lo, id_n, 1u);
-            }
-            tc_mma(d, a_lo, b_hi, id_n, 1u);
-          }
+        const uint64_t da = da0 + s * (uint32_t)(TC_A_STAGE >> 4), db = db0 + sb * (b_stage >> 4);
+        const uint32_t acc = it ? 1u : 0u;
+        if (wide) {
+          tc_mma(d, da, db, id_2n, acc), tc_mma(d, da + A_LO, db, id_n, 1u);
+          tc_mma(d, da + A_J, db + b_j, id_2n, 1u), tc_mma(d, da + A_J + A_LO, db + b_j, id_n, 1u);
+        } else {
+          tc_mma(d, da, db, id_n, acc), tc_mma(d, da, db + b_lo, id_n, 1u), tc_mma(d, da + A_LO, db, id_n, 1u);
+          tc_mma(d, da + A_J, db + b_j, id_n, 1u), tc_mma(d, da + A_J, db + b_j + b_lo, id_n, 1u), tc_mma(d, da + A_J + A_LO, db + b_j, id_n, 1u);
         }
         tc_commit(&empty_a[s]), tc_commit(&empty_b[sb]);  // arrive when the MMAs issued so far have completed: the stages may be refilled
         if (++s == a.sa) s = 0u, pa ^= 1u;
@@ -417,7 +432,7 @@ using namespace ieb;
 extern "C" size_t ie_b200_gemm_tc_scratch_bytes(uint32_t rows, uint32_t cols, uint32_t T) {
   const uint32_t nb = cols / 32u, nt = (T + TC_TOK - 1) / TC_TOK, splits = tc_splits(rows, nb, T);
   const size_t bp = (size_t)nt * nb * TC_TOK * TC_TOK_STAGE, part = splits > 1u ? (size_t)splits * T * rows * sizeof(float) : 0u;
-  const size_t scales = ((size_t)2 * nt * TC_TOK * sizeof(float) + 255u) & ~(size_t)255u;
+  const size_t scales = ((size_t)nt * TC_TOK * sizeof(float) + 255u) & ~(size_t)255u;
   return bp + part + scales + 512u;
 }
 
@@ -480,9 +495,11 @@ extern "C" int ie_b200_mat_tc_exp(int kind, const void *d_w, uint32_t rows, uint
   return IE_B200_OK;
 }
 
-extern "C" int ie_b200_gemm_tc(int kind, const void *d_w, uint32_t rows, uint32_t cols, int w_exp, const void *d_xq, float *d_y, const float *d_bias,
-                               const float *d_res, uint32_t T, size_t x_stride, size_t y_stride, size_t res_stride, void *d_scratch, size_t scratch_bytes,
-                               uint32_t *d_err, void *stream) {
+// act_ready: the scratch already holds the expanded activations of these Q8 rows (a call with the same columns and tokens was
+// launched on the stream before this one, and nothing has written to the scratch since).
+int ieb::gemm_tc_run(int kind, const void *d_w, uint32_t rows, uint32_t cols, int w_exp, const void *d_xq, float *d_y, const float *d_bias, const float *d_res,
+                     uint32_t T, size_t x_stride, size_t y_stride, size_t res_stride, void *d_scratch, size_t scratch_bytes, uint32_t *d_err, cudaStream_t st,
+                     bool act_ready) {
   if (!d_w || !d_xq || !d_y || !d_scratch) return fail(IE_B200_E_ARG, "ie_b200_gemm_tc: NULL pointer");
   if (kind != IE_B200_MAT_Q4 && kind != IE_B200_MAT_Q8 && kind != IE_B200_MAT_Q4K && kind != IE_B200_MAT_Q6K)
     return fail(IE_B200_E_ARG, "ie_b200_gemm_tc: matrix kind %d (Q4_0, Q8_0, Q4_K, Q6_K)", kind);
@@ -491,23 +508,23 @@ extern "C" int ie_b200_gemm_tc(int kind, const void *d_w, uint32_t rows, uint32_
   if (!aligned16(d_w) || !aligned16(d_xq) || (x_stride & 15u) || (y_stride & 3u) || (res_stride & 3u) || ((uintptr_t)d_scratch & 255u))
     return fail(IE_B200_E_ARG, "ie_b200_gemm_tc: the matrix and the Q8 rows must be 16-byte aligned, strides multiples of 4, the scratch 256-byte aligned");
   if (scratch_bytes < ie_b200_gemm_tc_scratch_bytes(rows, cols, T)) return fail(IE_B200_E_SIZE, "ie_b200_gemm_tc: scratch of %zu bytes, %zu needed", scratch_bytes, ie_b200_gemm_tc_scratch_bytes(rows, cols, T));
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   const uint32_t nb = cols / 32u, nt = (T + TC_TOK - 1) / TC_TOK, splits = tc_splits(rows, nb, T);
   if (w_exp < -100 || w_exp > 100) return fail(IE_B200_E_ARG, "ie_b200_gemm_tc: weight exponent %d", w_exp);
   uint8_t *bp = static_cast<uint8_t *>(d_scratch);
-  const size_t bp_bytes = ((size_t)nt * nb * TC_TOK * TC_TOK_STAGE + 255u) & ~(size_t)255u, sc_bytes = ((size_t)2 * nt * TC_TOK * sizeof(float) + 255u) & ~(size_t)255u;
-  float *tok_scale = reinterpret_cast<float *>(bp + bp_bytes), *tok_inv = tok_scale + (size_t)nt * TC_TOK;
+  const size_t bp_bytes = ((size_t)nt * nb * TC_TOK * TC_TOK_STAGE + 255u) & ~(size_t)255u, sc_bytes = ((size_t)nt * TC_TOK * sizeof(float) + 255u) & ~(size_t)255u;
+  float *tok_inv = reinterpret_cast<float *>(bp + bp_bytes);
   float *partial = splits > 1u ? reinterpret_cast<float *>(bp + bp_bytes + sc_bytes) : nullptr;
-  IEB_LAUNCH_PDL("tc_tokscale_kernel", tc_tokscale_kernel, dim3((T + 7u) / 8u), dim3(256), 0, st, static_cast<const uint8_t *>(d_xq), x_stride, T, nb,
-                 ldexpf(1.0f, -w_exp), tok_scale, tok_inv);
-  IEB_LAUNCH_PDL("tc_expand_kernel", tc_expand_kernel, dim3(nb, nt), dim3(256), 0, st, static_cast<const uint8_t *>(d_xq), x_stride, T, nb,
-                 static_cast<const float *>(tok_scale), bp);
+  if (!act_ready) {
+    // about four CTAs per SM, at least 32 blocks each
+    const uint32_t groups = (nt - 1u) * (TC_TOK / 8u) + tc_pad(T, nt - 1u) / 8u, parts = std::min((nb + 31u) / 32u, (4u * sm_count() + groups - 1u) / groups);
+    IEB_LAUNCH_PDL("tc_expand_kernel", tc_expand_kernel, dim3(groups, parts), dim3(256), 0, st, static_cast<const uint8_t *>(d_xq), x_stride, T, nb, tok_inv, bp);
+  }
   TcArgs a = {};
   a.w = static_cast<const uint8_t *>(d_w), a.rowb = row_bytes_of(kind, cols), a.rows = rows, a.nb = nb, a.T = T;
   a.blocks_per_split = (nb + splits - 1u) / splits;
   a.blocks_per_split = (a.blocks_per_split + 3u) & ~3u;  // whole raw stages
   a.bp = bp, a.y = d_y, a.bias = d_bias, a.res = d_res, a.ys = y_stride, a.rs = res_stride, a.partial = partial, a.err = d_err;
-  a.w_scale = ldexpf(1.0f, w_exp), a.tok_inv = tok_inv;
+  a.w_scale = ldexpf(1.0f, w_exp), a.w_inv = ldexpf(1.0f, -w_exp), a.tok_inv = tok_inv;
   const uint32_t used_splits = (nb + a.blocks_per_split - 1u) / a.blocks_per_split;
   const dim3 grid((rows + TC_ROWS - 1) / TC_ROWS, nt, partial ? used_splits : 1u);
   void (*k)(TcArgs) = kind == IE_B200_MAT_Q4 ? gemm_tc_kernel<IE_B200_MAT_Q4> : kind == IE_B200_MAT_Q8 ? gemm_tc_kernel<IE_B200_MAT_Q8>
@@ -529,4 +546,11 @@ extern "C" int ie_b200_gemm_tc(int kind, const void *d_w, uint32_t rows, uint32_
     IEB_LAUNCH_PDL("tc_reduce_kernel", tc_reduce_kernel, dim3((rows + 255u) / 256u, T), dim3(256), 0, st, static_cast<const float *>(partial), used_splits, T, rows, d_y,
                    d_bias, d_res, y_stride, res_stride);
   return IE_B200_OK;
+}
+
+extern "C" int ie_b200_gemm_tc(int kind, const void *d_w, uint32_t rows, uint32_t cols, int w_exp, const void *d_xq, float *d_y, const float *d_bias,
+                               const float *d_res, uint32_t T, size_t x_stride, size_t y_stride, size_t res_stride, void *d_scratch, size_t scratch_bytes,
+                               uint32_t *d_err, void *stream) {
+  return gemm_tc_run(kind, d_w, rows, cols, w_exp, d_xq, d_y, d_bias, d_res, T, x_stride, y_stride, res_stride, d_scratch, scratch_bytes, d_err,
+                     static_cast<cudaStream_t>(stream), false);
 }
