@@ -415,6 +415,32 @@ __global__ void __launch_bounds__(256) tc_reduce_kernel(const float *partial, ui
   }
 }
 
+// The same four rows per thread (rows a multiple of 4, 16-byte aligned rows): all splits' loads on their way at once.
+__global__ void __launch_bounds__(128) tc_reduce4_kernel(const float *partial, uint32_t splits, uint32_t T, uint32_t rows, float *y, const float *bias,
+                                                         const float *res, size_t ys, size_t rs) {
+  pdl_prologue();
+  const uint32_t n = blockIdx.y, r = 4u * (blockIdx.x * 128u + threadIdx.x);
+  if (r >= rows) return;
+  const float4 *src = reinterpret_cast<const float4 *>(partial + (size_t)n * rows + r);
+  const size_t step = (size_t)T * rows / 4u;
+  float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  for (uint32_t s0 = 0; s0 < splits; s0 += 4u) {
+    float4 p[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++)
+      if (s0 + k < splits) p[k] = __ldcg(src + (s0 + k) * step);
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++)
+      if (s0 + k < splits) o.x = __fadd_rn(o.x, p[k].x), o.y = __fadd_rn(o.y, p[k].y), o.z = __fadd_rn(o.z, p[k].z), o.w = __fadd_rn(o.w, p[k].w);
+  }
+  if (bias) o.x = __fadd_rn(o.x, bias[r]), o.y = __fadd_rn(o.y, bias[r + 1]), o.z = __fadd_rn(o.z, bias[r + 2]), o.w = __fadd_rn(o.w, bias[r + 3]);
+  if (res) {
+    const float4 v = *reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(res) + rs * n + 4u * (size_t)r);
+    o.x = __fadd_rn(v.x, o.x), o.y = __fadd_rn(v.y, o.y), o.z = __fadd_rn(v.z, o.z), o.w = __fadd_rn(v.w, o.w);
+  }
+  *reinterpret_cast<float4 *>(reinterpret_cast<char *>(y) + ys * n + 4u * (size_t)r) = o;
+}
+
 static uint32_t tc_splits(uint32_t rows, uint32_t nb, uint32_t T) {
   const uint32_t ctas = ((rows + TC_ROWS - 1) / TC_ROWS) * ((T + TC_TOK - 1) / TC_TOK);
   const uint32_t sms = (uint32_t)sm_count();
@@ -542,7 +568,11 @@ int ieb::gemm_tc_run(int kind, const void *d_w, uint32_t rows, uint32_t cols, in
   const uint32_t smem = smem_of(a.sa, a.sb);
   if (int r = ensure_dynamic_smem(reinterpret_cast<const void *>(k), smem)) return r;
   IEB_LAUNCH_PDL("gemm_tc_kernel", k, grid, dim3(TC_THREADS), smem, st, a);
-  if (partial)
+  const bool vec = rows % 4u == 0 && !(((uintptr_t)d_y | y_stride | (uintptr_t)d_res | res_stride | (uintptr_t)partial) & 15u);
+  if (partial && vec)
+    IEB_LAUNCH_PDL("tc_reduce4_kernel", tc_reduce4_kernel, dim3((rows / 4u + 127u) / 128u, T), dim3(128), 0, st, static_cast<const float *>(partial), used_splits, T,
+                   rows, d_y, d_bias, d_res, y_stride, res_stride);
+  else if (partial)
     IEB_LAUNCH_PDL("tc_reduce_kernel", tc_reduce_kernel, dim3((rows + 255u) / 256u, T), dim3(256), 0, st, static_cast<const float *>(partial), used_splits, T, rows, d_y,
                    d_bias, d_res, y_stride, res_stride);
   return IE_B200_OK;

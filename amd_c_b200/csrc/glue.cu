@@ -152,6 +152,47 @@ __global__ void __launch_bounds__(256) swiglu_il_kernel(const float *gu, float *
   if (q && 32u * blk + 32u <= n) quant_block_warp(v, row_ptr(q, qs, t), n / 32u, blk, lane);
 }
 
+// The same for whole blocks and 16-byte aligned rows: four outputs per thread, eight threads per block (two 16-byte loads, one
+// store and three exchanges instead of five; the bound for a chunk is the pass over memory: 256 x 18944, 27 us with one output per thread).
+__global__ void __launch_bounds__(256) swiglu_il4_kernel(const float *gu, float *h, uint32_t n, uint8_t *q, size_t gs, size_t hs, size_t qs) {
+  pdl_prologue();
+  const uint32_t t = blockIdx.y, i = 4u * (blockIdx.x * 256u + threadIdx.x);
+  const bool ok = i < n;
+  float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  if (ok) {
+    const float4 *src = reinterpret_cast<const float4 *>(row_ptr(gu, gs, t) + 2u * (size_t)i);
+    const float4 p0 = src[0], p1 = src[1];
+    const float g[4] = {p0.x, p0.z, p1.x, p1.z}, u[4] = {p0.y, p0.w, p1.y, p1.w};
+#pragma unroll
+    for (int c = 0; c < 4; c++) v[c] = __fmul_rn(__fdiv_rn(g[c], __fadd_rn(1.0f, expf(-g[c]))), u[c]);
+    *reinterpret_cast<float4 *>(row_ptr(h, hs, t) + i) = make_float4(v[0], v[1], v[2], v[3]);
+  }
+  if (!q) return;
+  float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+  const float d = __fdiv_rn(amax, 127.0f);
+  const Q8Div qd = q8_div(d);
+  uint32_t pk = 0u;
+  int sum = 0;
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    const int x = q8_round(v[c], qd);
+    sum += x;
+    pk |= (uint32_t)(x & 255) << (8 * c);
+  }
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+  if (ok) {
+    uint8_t *qt = row_ptr(q, qs, t);
+    *reinterpret_cast<uint32_t *>(qt + i) = pk;
+    if ((threadIdx.x & 7u) == 0u) {
+      reinterpret_cast<float *>(qt + n)[i / 32u] = d;
+      reinterpret_cast<int *>(qt + n + n / 8u)[i / 32u] = sum;
+    }
+  }
+}
+
 // ---- RoPE of q and k in place, then K/V of the position into the cache ----
 // Cache layout: [kv head][row][hd], row = position % kv_len.
 template <typename KV>
@@ -424,6 +465,11 @@ extern "C" int ie_b200_swiglu_il(const float *d_gu, float *d_h, uint32_t n, void
   if (((uintptr_t)d_gu & 7u) || (gu_stride & 7u)) return fail(IE_B200_E_ARG, "ie_b200_swiglu_il: the gate / up pairs must be 8-byte aligned");
   if (n == 0 || T == 0) return IE_B200_OK;
   if (T > 65535u) return fail(IE_B200_E_SIZE, "ie_b200_swiglu_il: T %u > 65535", T);
+  if (n % 32u == 0 && !(((uintptr_t)d_gu | gu_stride | (uintptr_t)d_h | h_stride) & 15u) && !(((uintptr_t)d_q | q_stride) & 3u)) {
+    IEB_LAUNCH_PDL("swiglu_il4_kernel", swiglu_il4_kernel, dim3((n / 4u + 255u) / 256u, T), dim3(256), 0, static_cast<cudaStream_t>(stream), d_gu, d_h, n,
+                   static_cast<uint8_t *>(d_q), gu_stride, h_stride, q_stride);
+    return IE_B200_OK;
+  }
   const uint32_t nblk = (n + 31u) / 32u;
   IEB_LAUNCH_PDL("swiglu_il_kernel", swiglu_il_kernel, dim3((nblk + 7u) / 8u, T), dim3(256), 0, static_cast<cudaStream_t>(stream), d_gu, d_h, n,
                  static_cast<uint8_t *>(d_q), gu_stride, h_stride, q_stride);

@@ -641,7 +641,8 @@ def test_gemm_matches_gemv(ora, cuda, typ, rows, cols, T):
                                              (synth.GGML_Q6_K, 512, 1024, 131), (synth.GGML_Q4_K, 96, 512, 40), (synth.GGML_Q4_0, 77, 192, 33),
                                              (synth.GGML_Q4_0, 130, 320, 20), (synth.GGML_Q4_0, 5000, 4096, 300), (synth.GGML_Q6_K, 300, 18944, 64),
                                              (synth.GGML_Q4_K, 9000, 3584, 256), (synth.GGML_Q4_0, 1, 64, 1), (synth.GGML_Q8_0, 1000, 4096, 100),
-                                             (synth.GGML_Q8_0, 77, 192, 33), (synth.GGML_Q8_0, 4096, 14336, 256)])
+                                             (synth.GGML_Q8_0, 77, 192, 33), (synth.GGML_Q8_0, 4096, 14336, 256), (synth.GGML_Q4_0, 1001, 4096, 40),
+                                             (synth.GGML_Q6_K, 130, 2048, 129), (synth.GGML_Q8_0, 300, 32 * 38, 128)])
 def test_gemm_tc_matches_gemv(ora, cuda, typ, rows, cols, T):
     """The prompt-chunk GEMM on tcgen05 / tensor memory (both operands as two half-precision terms, fp32 accumulation over the
     whole K in tensor memory) against the multi-token GEMV, which is bit-exact with the CPU reference: 1e-5 of the largest
@@ -972,6 +973,29 @@ def test_swiglu_inside_the_gemvs(ora, cuda, lib, typ, ffn, dim):
     assert (hq.cpu().numpy() == want_q).all()
     kd, dw, ds = ora.repack(synth.GGML_Q4_0, down, dim, ffn)
     assert (bits(y.cpu().numpy()) == bits(ora.gemv(kd, dw, ds, dim, ffn, want_q, res=res))).all()
+
+
+@pytest.mark.parametrize("n,T", [(32, 1), (1056, 3), (14336, 1), (18944, 7)])
+def test_swiglu_interleaved_wide_and_narrow(cuda, lib, n, T):
+    """The four-outputs-per-thread form (rows of whole blocks, 16-byte aligned) against the one-output form, which a result 4
+    bytes off the alignment takes: the same bits, values and Q8 copies, blocks of zeros and infinities among them."""
+    import torch
+
+    from amd_c_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    gu = torch.randn((T, 2 * n), generator=gen, device=cuda) * 4
+    gu[0, :64] = 0.0
+    if n > 64:
+        gu[T - 1, 70], gu[T - 1, 100] = float("inf"), -float("inf")
+    nb = n // 32
+    h, q = torch.empty((T, n), device=cuda), torch.zeros((T, 40 * nb), dtype=torch.uint8, device=cuda)
+    flat, q2 = torch.empty(T * n + 1, device=cuda), torch.zeros((T, 40 * nb), dtype=torch.uint8, device=cuda)
+    K.check(lib.ie_b200_swiglu_il(gu.data_ptr(), h.data_ptr(), n, q.data_ptr(), T, 8 * n, 4 * n, 40 * nb, None))
+    K.check(lib.ie_b200_swiglu_il(gu.data_ptr(), flat.data_ptr() + 4, n, q2.data_ptr(), T, 8 * n, 4 * n, 40 * nb, None))
+    torch.cuda.synchronize()
+    assert torch.equal(h.view(-1).view(torch.int32), flat[1:].view(torch.int32))
+    assert torch.equal(q, q2)
 
 
 def test_swiglu_interleaved_equals_planar(cuda, lib):
