@@ -3,9 +3,11 @@
 //
 // The block dots come from the int8 tensor cores: one mma.sync m16n8k32 is the exact int32 dot of one 32-weight block for 16
 // rows x 8 tokens. With dp4a per token the kernel was bound by instruction issue; here the work per block and token is the
-// scaling in fp32, two tokens per instruction (f32x2). Measured, before -> now, 6 tokens: 28672 x 4096 Q4_0 58 -> 24 us, 4096 x
-// 14336 Q4_0 49 -> 18, 128256 x 4096 Q4_0 222 -> 85, 37888 x 3584 Q4_K 86 -> 32, 3584 x 18944 Q6_K 88 -> 31; 2 tokens: 41 -> 24,
-// 35 -> 20, 155 -> 86, 55 -> 32, 58 -> 29; 16 tokens: 154 -> 37, 101 -> 31, 646 -> 133, 197 -> 43, 185 -> 52.
+// scaling in fp32, two tokens per instruction (f32x2). What bounds it now is still issue: about 55 instructions per 16 rows x one
+// block x 8 tokens, 16 warps of 128 registers per SM (24 warps of 80 were slower: 28672 x 4096 24 against 22 us).
+// Measured, dp4a -> now, 6 tokens: 28672 x 4096 Q4_0 58 -> 22 us, 4096 x 14336 Q4_0 49 -> 16, 128256 x 4096 Q4_0 222 -> 81, 37888 x
+// 3584 Q4_K 86 -> 29, 3584 x 18944 Q6_K 88 -> 28; 2 tokens: 41 -> 21, 35 -> 14, 155 -> 80, 55 -> 28, 58 -> 26; 16 tokens: 154 -> 35,
+// 101 -> 30, 646 -> 126, 197 -> 42, 185 -> 50.
 //
 // Order: the one-token GEMV gives lane l of a warp the blocks l, l + 32, ... in order and adds the 32 lane sums by a tree
 // (16, 8, 4, 2, 1). Warp w of the eight that share a 16-row tile keeps the sums of "lanes" 4 w .. 4 w + 3 in registers (four
@@ -22,9 +24,9 @@
 
 namespace ieb {
 
-constexpr int GT_WARPS = 16, GT_THREADS = GT_WARPS * 32;
+constexpr int GT_WARPS = 16, GT_THREADS = GT_WARPS * 32;       // two 16-row tiles of eight warps each
 constexpr uint32_t GT_RED_LANE = 176;                          // floats per lane sum of a tile: 8 tokens x 20 (16 rows, padded), 16 mod 32
-constexpr uint32_t GT_RED = 2u * 32u * GT_RED_LANE * 4u;       // both tiles of the CTA
+constexpr uint32_t GT_RED = 32u * GT_RED_LANE * 4u;            // of one tile
 constexpr uint32_t GT_SMEM = 227u * 1024u;
 constexpr int GT_BIAS = 0x4B400000;                            // 1.5 * 2^23: an int32 |n| < 2^22 added to these bits is the float 12582912 + n
 
@@ -33,6 +35,10 @@ template <> struct GtKind<IE_B200_MAT_Q4> { static constexpr uint32_t DS = 64, S
 template <> struct GtKind<IE_B200_MAT_Q8> { static constexpr uint32_t DS = 64, SMAX = 4; };
 template <> struct GtKind<IE_B200_MAT_Q4K> { static constexpr uint32_t DS = 64, SMAX = 6; };
 template <> struct GtKind<IE_B200_MAT_Q6K> { static constexpr uint32_t DS = 96, SMAX = 4; };
+
+// Stages of a warp's ring: as many as leave room for the activations.
+template <int KIND, int NT>
+constexpr int GT_STAGES = NT == 1 ? (int)GtKind<KIND>::SMAX : 4;
 
 struct GtArgs {
   const uint8_t *w;
@@ -185,13 +191,13 @@ __device__ __forceinline__ void gt_step(const uint8_t *stp, uint32_t b0, const u
 
 template <int KIND, int NT>
 __global__ void __launch_bounds__(GT_THREADS, 1) gemv_tokens_kernel(const GtArgs a) {
-  constexpr int S = NT == 1 ? (int)GtKind<KIND>::SMAX : 4;
+  constexpr int S = GT_STAGES<KIND, NT>;
   constexpr uint32_t STAGE = RS_BYTES<KIND>, DS = GtKind<KIND>::DS;
   extern __shared__ __align__(128) uint8_t smem_gt[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, w = warp & 7, half = warp >> 3;
   uint8_t *ring = smem_gt + (uint32_t)warp * S * STAGE;
   float *red = reinterpret_cast<float *>(smem_gt + GT_WARPS * S * STAGE) + half * 32u * GT_RED_LANE;
-  uint8_t *sB = smem_gt + GT_WARPS * S * STAGE + GT_RED, *sD = sB + (size_t)a.P * NT * 256u;
+  uint8_t *sB = smem_gt + GT_WARPS * S * STAGE + 2u * GT_RED, *sD = sB + (size_t)a.P * NT * 256u;
   pdl_launch_dependents();
   const uint32_t nb = a.nb, tiles = (a.rows + 15u) / 16u, t0 = blockIdx.y * 8u * NT;
   // tiles of this half of the CTA: slot, slot + 2 gridDim.x, ... (the first halves of all CTAs come first)
@@ -199,11 +205,13 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemv_tokens_kernel(const GtArgs
   const uint32_t mine = slot < tiles ? (tiles - slot + stride - 1u) / stride : 0u, most = (tiles - blockIdx.x + stride - 1u) / stride;
   const uint32_t steps = nb > 4u * w ? (nb - 4u * w + 31u) / 32u : 0u;  // of this warp, per tile
   const uint32_t items = mine * steps;
-  // next item to ask for
+  // next item to ask for; the rows' addresses are worked out once per tile (rows past the end: copies that are not stored)
+  RsRows<KIND> rr;
   uint32_t in = 0, it_tile = slot, it_j = 0, it_stage = 0;
   auto issue = [&]() {
     if (in < items) {
-      rs_issue<KIND>(a.w, a.rowb, a.rows, nb, rs_smem(ring + it_stage * STAGE), it_tile * 16u, 32u * it_j + 4u * w, lane);
+      if (it_j == 0u) rr.set(a.w, a.rowb, a.rows, nb, it_tile * 16u, lane);
+      rs_issue_rows<KIND>(rr, nb, rs_smem(ring + it_stage * STAGE), 32u * it_j + 4u * w, lane);
       in++;
       if (++it_j == steps) it_j = 0, it_tile += stride;
     }
@@ -283,7 +291,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemv_tokens_kernel(const GtArgs
 
 template <int KIND, int NT>
 static int launch_tokens(GtArgs a, cudaStream_t st) {
-  constexpr uint32_t S = NT == 1 ? GtKind<KIND>::SMAX : 4u, fixed = GT_WARPS * S * RS_BYTES<KIND> + GT_RED, per = NT * (256u + GtKind<KIND>::DS);
+  constexpr uint32_t fixed = 2u * (8u * GT_STAGES<KIND, NT> * RS_BYTES<KIND> + GT_RED), per = NT * (256u + GtKind<KIND>::DS);
   // the fewest phases whose activations fit beside the rings, all of about the same length
   const uint32_t cap = (GT_SMEM - fixed) / per / 32u * 32u, up = (a.nb + 31u) & ~31u, phases = (up + cap - 1u) / cap;
   static_assert((GT_SMEM - fixed) / per >= 32u, "a phase is at least 32 blocks");
@@ -297,9 +305,21 @@ static int launch_tokens(GtArgs a, cudaStream_t st) {
   return IE_B200_OK;
 }
 
+// Sixteen tokens per pass, the last eight or fewer with one token tile.
 template <int KIND>
-static int pick_tokens(const GtArgs &a, cudaStream_t st) {
-  return a.T <= 8u ? launch_tokens<KIND, 1>(a, st) : launch_tokens<KIND, 2>(a, st);
+static int pick_tokens(GtArgs a, cudaStream_t st) {
+  const uint32_t tail = a.T % 16u, two = tail > 8u ? a.T : a.T - tail;  // tokens worked sixteen at a time
+  const uint32_t all = a.T;
+  if (two) {
+    a.T = two;
+    if (int r = launch_tokens<KIND, 2>(a, st)) return r;
+  }
+  if (two == all) return IE_B200_OK;
+  a.T = all - two;
+  a.xq += (size_t)two * a.xs;
+  a.y = reinterpret_cast<float *>(reinterpret_cast<char *>(a.y) + (size_t)two * a.ys);
+  if (a.res) a.res = reinterpret_cast<const float *>(reinterpret_cast<const char *>(a.res) + (size_t)two * a.rs);
+  return launch_tokens<KIND, 1>(a, st);
 }
 
 // y[t] = W x[t] (+ bias) (+ res[t]) for T >= 2 tokens; the checks are ie_b200_gemv's.

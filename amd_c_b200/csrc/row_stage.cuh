@@ -84,4 +84,51 @@ __device__ __forceinline__ void rs_issue(const uint8_t *w, size_t rowb, uint32_t
   }
 }
 
+// The same stage with the addresses of the rows a lane copies from kept for a whole tile. Rows past the matrix give a copy of its
+// last row (the caller does not store their results).
+template <int KIND>
+struct RsRows {
+  static constexpr int N = KIND == IE_B200_MAT_Q8 ? 4 : 2;
+  const uint8_t *rp[N];  // the pieces' rows, at the lane's piece
+  const uint8_t *hp;     // Q6_K: the high bits of row lane / 2
+  const uint8_t *sp;     // lanes 0..15: the scale fields of row `lane`
+  __device__ __forceinline__ void set(const uint8_t *w, size_t rowb, uint32_t rows, uint32_t nb, uint32_t row0, int lane) {
+#pragma unroll
+    for (uint32_t k = 0; k < N; k++) {
+      const uint32_t r = KIND == IE_B200_MAT_Q8 ? (uint32_t)(lane >> 3) + 4u * k : (uint32_t)(lane >> 2) + 8u * k;
+      rp[k] = w + (size_t)min(row0 + r, rows - 1u) * rowb + 16u * (lane & (KIND == IE_B200_MAT_Q8 ? 7u : 3u));
+    }
+    if (KIND == IE_B200_MAT_Q6K) hp = w + (size_t)min(row0 + ((uint32_t)lane >> 1), rows - 1u) * rowb + 16u * (size_t)nb + 16u * (lane & 1u);
+    sp = w + (size_t)min(row0 + (lane & 15u), rows - 1u) * rowb + (KIND == IE_B200_MAT_Q8 ? 32u : KIND == IE_B200_MAT_Q6K ? 24u : 16u) * (size_t)nb;
+  }
+};
+template <int KIND>
+__device__ __forceinline__ void rs_issue_rows(const RsRows<KIND> &rr, uint32_t nb, uint32_t st, uint32_t b0, int lane) {
+  if (KIND == IE_B200_MAT_Q8) {
+    const uint32_t c = lane & 7u;
+#pragma unroll
+    for (uint32_t k = 0; k < 4; k++) {
+      const uint32_t r = (uint32_t)(lane >> 3) + 4u * k;
+      rs_cp<16>(st + r * 128u + ((c ^ (r & 7u)) << 4), rr.rp[k] + 32u * (size_t)b0, b0 + (c >> 1) < nb);
+    }
+  } else {
+    const uint32_t c = lane & 3u;
+#pragma unroll
+    for (uint32_t k = 0; k < 2; k++) {
+      const uint32_t r = (uint32_t)(lane >> 2) + 8u * k;
+      rs_cp<16>(st + r * 64u + ((c ^ ((r >> 1) & 3u)) << 4), rr.rp[k] + 16u * (size_t)b0, b0 + c < nb);
+    }
+  }
+  if (KIND == IE_B200_MAT_Q6K) rs_cp<16>(st + 1024u + 16u * lane, rr.hp + 8u * (size_t)b0, true);
+  if (lane < 16) {
+    if (KIND == IE_B200_MAT_Q4) rs_cp<8>(st + 1024u + 8u * lane, rr.sp + 2u * b0, true, 2u * (nb - b0));
+    if (KIND == IE_B200_MAT_Q8) rs_cp<8>(st + 2048u + 8u * lane, rr.sp + 2u * b0, true, 2u * (nb - b0));
+    if (KIND == IE_B200_MAT_Q4K) rs_cp<16>(st + 1024u + 16u * lane, rr.sp + 16u * (b0 >> 3), true);
+    if (KIND == IE_B200_MAT_Q6K) {
+      rs_cp<8>(st + 1536u + 8u * lane, rr.sp + 2u * b0, true);
+      rs_cp<4>(st + 1664u + 4u * lane, rr.sp + 2u * (size_t)nb + ((2u * (b0 >> 3)) & ~3u), true);
+    }
+  }
+}
+
 }  // namespace ieb
