@@ -140,10 +140,17 @@ int attn_decode_fused(const float *d_q, const float *d_k, const float *d_v, void
 // Can the one-token decode GEMV take this matrix?
 static bool stream_ok(const EMat &m) { return gemv_direct_ok(m.kind, m.cols); }
 
-// Does the tcgen05 GEMM run op o over T tokens?
+// A few tokens above sixteen: two passes of the multi-token GEMV over the weights, or one of the tcgen05 GEMM, whose products cost
+// about the same from 17 to 100 tokens? Up to 24 tokens (the second pass has one token tile) the GEMV is ahead where its
+// activations stay in shared memory: 28672 x 4096 Q4_0 56 .. 58 against 71 us, 6144 x 4096 20 .. 21 / 23, 2048 x 2048 Q8_0 8 / 13,
+// 37888 x 3584 Q4_K 70 .. 72 / 76; not for long rows (4096 x 14336 42 .. 47 / 39 .. 40, 2048 x 8192 Q8_0 21 .. 23 / 19 .. 20) nor for
+// Q6_K, two tensor products per block (2048 x 4096 15 .. 16 / 15); at 28 tokens it is level (66 / 71, 20 / 19, 83 / 77).
+static bool few_tokens(const EMat &m, uint32_t T) { return T <= 24u && m.cols <= 6144u && m.kind != IE_B200_MAT_Q6K; }
+
+// Does the tcgen05 GEMM run op o over T tokens? (From the reference's threshold on, src/hip.c:965.)
 static bool tc_gemm(const ie_b200_engine *e, const ie_b200_op &o, uint32_t T) {
   return o.kind == IE_B200_OP_GEMV && o.mat >= 0 && (size_t)o.mat < e->mats.size() && T >= 17 && e->mats[o.mat].kind != IE_B200_MAT_F32 && !e->no_gemm &&
-         !e->gemm_mma && o.a_stride % 16u == 0;
+         !e->gemm_mma && o.a_stride % 16u == 0 && !few_tokens(e->mats[o.mat], T);
 }
 // Are the expanded activations that GEMM op p left in the scratch also those of op o, launched right after it with nothing
 // between them (q, k and v of a layer)? The same Q8 rows, and p's result does not lie over them: all of it before or behind
@@ -187,7 +194,7 @@ static int launch_op(ie_b200_engine *e, const ie_b200_op &o, uint32_t t0, uint32
       // a prompt chunk (the reference's threshold, src/hip.c:965): the tensor-core GEMM reads the weights once per 128 tokens
       const bool tc_ok = !e->gemm_mma && o.a_stride % 16u == 0;
       // (Q8_0 has no mma.sync form: where the tcgen05 kernel cannot run it takes the multi-token GEMV below, 8 tokens per pass)
-      if (T >= 17 && m.kind != IE_B200_MAT_F32 && !e->no_gemm && (tc_ok || m.kind != IE_B200_MAT_Q8)) {
+      if (T >= 17 && m.kind != IE_B200_MAT_F32 && !e->no_gemm && (tc_ok || m.kind != IE_B200_MAT_Q8) && !(tc_ok && few_tokens(m, T))) {
         if (tc_ok) {  // tcgen05 / tensor memory
           EMat &mm = e->mats[o.mat];
           // (normally done by prepare_chunks before anything of the run is enqueued; here for callers that enqueue ranges themselves)
