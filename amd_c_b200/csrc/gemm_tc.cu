@@ -20,9 +20,8 @@
 //                residual and store token rows (32 consecutive rows per warp store: coalesced).
 // Two rings, handed over with mbarriers (full: sixteen producer warps / the bulk copy's bytes; empty: tcgen05.commit): 32 KB of
 // weights and the tokens' 128 bytes each of activations per 32-column stage, as many stages as fit.
-// Matrices with few rows
-// (3584 x 18944: 14 CTAs) are split along K over grid.z, every split writing its partial sums to scratch, which a second
-// kernel adds in split order (deterministic). Every mbarrier wait is bounded by wall time and reports through the device
+// Matrices with few rows (3584 x 18944: 14 CTAs) are split along K over grid.z, every split writing its partial sums to
+// scratch, which a second kernel adds in split order (deterministic). Every mbarrier wait is bounded by wall time and reports through the device
 // error word; tensor memory is freed on every path.
 //
 // Half precision has a narrow exponent range, so both sides are scaled by exact powers of two before they are split (a value
@@ -36,7 +35,8 @@
 // products per weight and token: 126 us of f16 work for the 37888 rows at the measured bf16 burst rate).
 //
 // Result: equal to the one-token GEMV (which is bit-exact with the CPU) to fp32 rounding: not bit for bit, as the
-// reference's GEMM against its GEMV.
+// reference's GEMM against its GEMV. Relative error against 64 bits (2-norm; the f32 accumulation dominates): Q4_0 4096 columns
+// 9.0e-7, 14336 3.0e-6, Q4_K 3584 9.8e-7, Q6_K 18944 4.5e-6 above 128 tokens; with two accumulators 5.9e-7, 1.9e-6, 6.7e-7, 3.0e-6.
 #include <cuda_fp16.h>
 #include <math.h>
 #include <string.h>
