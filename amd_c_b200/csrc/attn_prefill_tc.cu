@@ -303,7 +303,12 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
         ok = __all_sync(0xFFFFFFFFu, mbar_wait(pair, n & 1u, &s_abort));
         l += x[(half ^ 1u) * 128u + rl];
       }
-      if (ok) {
+      if (ok && n == 0u) {
+        // A split without blocks for this tile (the splits are dealt for the whole chunk's positions): an empty record, whose row the
+        // merge does not read. Nothing is staged: no wait of this path says that the other warps have stored their part of Q.
+        if (real && half == 0u)
+          *reinterpret_cast<float2 *>(a.ml + (split * (size_t)a.T * a.n_head + (size_t)tok * a.n_head + head) * 2u) = make_float2(-INFINITY, 0.0f);
+      } else if (ok) {
         tc_fence_after();
         constexpr uint32_t UN = HD / 8;  // 16-byte units of the half row that a warp writes
         const uint32_t nbq = a.n_head * HD / 32u;
@@ -313,12 +318,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
 #pragma unroll 1
         for (int c = 0; c < HD / 64; c++) {
           uint32_t v[32];
-#pragma unroll
-          for (int i = 0; i < 32; i++) v[i] = 0u;
-          if (n > 0u) {
-            tc_ld32(o_col + 32u * c, v);
-            tc_wait_ld();
-          }
+          tc_ld32(o_col + 32u * c, v);
+          tc_wait_ld();
 #pragma unroll
           for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * inv);
 #pragma unroll
@@ -349,7 +350,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
         }
         if (a.part && real && half == 0u) {
           float *ml = a.ml + (split * all + (size_t)tok * a.n_head + head) * 2u;
-          ml[0] = n > 0u ? m : -INFINITY, ml[1] = n > 0u ? l : 0.0f;
+          ml[0] = m, ml[1] = l;
         }
         __syncwarp();
         const uint32_t u = (uint32_t)lane % UN;
@@ -481,7 +482,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
   if (warp == PT_SOFT_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
 
-// The splits' records of a (token, head) row -> its output and Q8 copy: hd / 4 lanes per row, four floats each.
+// The splits' records of a (token, head) row -> its output and Q8 copy: hd / 4 lanes per row, four floats each. A record (-inf, 0)
+// is of a split that holds nothing the row sees: its row is not read (it may never have been written).
 template <int HD>
 __global__ void __launch_bounds__(256) attn_prefill_merge_kernel(const float *part, const float *ml, uint32_t splits, uint32_t T, uint32_t n_head, float *out,
                                                                  uint8_t *oq, size_t out_stride, size_t oq_stride, uint32_t wide) {
@@ -496,8 +498,9 @@ __global__ void __launch_bounds__(256) attn_prefill_merge_kernel(const float *pa
 #pragma unroll 4
   for (uint32_t s = 0; s < splits; s++) {
     const float2 e = *reinterpret_cast<const float2 *>(ml + 2u * ((size_t)s * all + row));
+    if (e.x == -INFINITY && e.y == 0.0f) continue;
     const float4 v = *reinterpret_cast<const float4 *>(part + ((size_t)s * all + row) * HD + col);
-    const float w = ex2(e.x - M);  // 0 for a split that saw nothing (its row is zero)
+    const float w = ex2(e.x - M);
     L = fmaf(w, e.y, L);
     acc.x = fmaf(w, v.x, acc.x), acc.y = fmaf(w, v.y, acc.y), acc.z = fmaf(w, v.z, acc.z), acc.w = fmaf(w, v.w, acc.w);
   }

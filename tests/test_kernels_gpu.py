@@ -753,6 +753,46 @@ def test_attention_prefill_tiles(cuda, n_head, n_kv, hd, T, pos0, split):
     assert (oq == K.quant_q8(out)).all()
 
 
+@pytest.mark.parametrize("n_head,n_kv,hd,T,pos0", [(28, 4, 128, 64, 1000), (8, 1, 64, 96, 1000)])
+def test_attention_prefill_empty_splits(cuda, lib, n_head, n_kv, hd, T, pos0):
+    """More splits of the positions than the first row tiles have blocks of 128: the records of the splits without blocks are not
+    read, whatever the scratch held before (NaN here), and a NaN in the query rows of one token stays in that token's row. All
+    other rows bit for bit those of the run without it."""
+    import torch
+
+    from amd_c_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    n, w = pos0 + T, n_head * hd
+    kc, vc = (torch.randn((n_kv, n, hd), generator=gen, device=cuda).half() for _ in range(2))
+    q = torch.randn((T, w), generator=gen, device=cuda)
+    pos = torch.tensor([pos0], dtype=torch.int32, device=cuda)
+    scratch = torch.empty(lib.ie_b200_attn_prefill_scratch_bytes(n_head, hd, T) // 4, device=cuda)
+    err = torch.zeros(1, dtype=torch.int32, device=cuda)
+
+    def run(qq, positions):
+        out = torch.empty((T, w), device=cuda)
+        scratch.fill_(float("nan"))
+        K.check(lib.ie_b200_attn_prefill_split(qq.data_ptr(), kc.data_ptr(), vc.data_ptr(), out.data_ptr(), None, pos.data_ptr(), n_head, n_kv, hd, n, T,
+                                               4 * w, 4 * w, 0, positions, scratch.data_ptr(), err.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        return out
+
+    # (`positions` only sizes the grid: 4 n asks for more splits than there are blocks of positions at all)
+    for positions in (n, 4 * n):
+        want = run(q, positions)
+        assert torch.isfinite(want).all()
+        one, _ = K.attn_prefill(q, kc, vc, pos, n_head, n_kv, hd)
+        assert (want - one).abs().max() <= 1e-5 * one.abs().max()  # two summation orders of fp32 sums
+        for t in (0, 5, T - 1):
+            bad = q.clone()
+            bad[t, : hd] = float("nan")
+            got = run(bad, positions)
+            rows = torch.arange(T, device=cuda) != t
+            assert torch.equal(got[rows].view(torch.int32), want[rows].view(torch.int32)), t
+            assert torch.isnan(got[t, :hd]).all() and torch.equal(got[t, hd:].view(torch.int32), want[t, hd:].view(torch.int32))
+    assert int(err.item()) == 0
+
+
 @pytest.mark.parametrize("typ,rows,cols,T", [(synth.GGML_Q4_0, 130, 1024, 11), (synth.GGML_Q4_K, 77, 512, 16), (synth.GGML_Q6_K, 40, 18944, 5),
                                              (synth.GGML_Q4_0, 9, 64, 2), (synth.GGML_Q8_0, 130, 1024, 11), (synth.GGML_Q8_0, 40, 4096, 16)])
 def test_gemv_several_tokens_one_pass(ora, cuda, typ, rows, cols, T):
