@@ -564,6 +564,13 @@ static int launch_pt(const PtArgs &a, const void *kc, const void *vc, uint32_t s
 int attn_prefill_tc(const float *d_q, const void *d_kc, const void *d_vc, float *d_out, void *d_oq, const uint32_t *d_pos, uint32_t n_head, uint32_t n_kv,
                     uint32_t hd, uint32_t kv_len, uint32_t T, size_t q_stride, size_t out_stride, size_t oq_stride, uint32_t positions, float *d_scratch,
                     uint32_t *d_err, cudaStream_t st) {
+  if (!d_q || !d_kc || !d_vc || !d_out || !d_pos) return fail(IE_B200_E_ARG, "ie_b200_attn_prefill: NULL pointer");
+  if (n_kv == 0 || n_head % n_kv) return fail(IE_B200_E_SIZE, "ie_b200_attn_prefill: %u heads over %u KV heads", n_head, n_kv);
+  if (hd != 64 && hd != 128) return fail(IE_B200_E_SIZE, "ie_b200_attn_prefill: head dim %u (64, 128; half-precision cache)", hd);
+  if (!aligned16(d_kc) || !aligned16(d_vc) || ((uintptr_t)d_q & 7u) || (q_stride & 7u) || (d_scratch && !aligned16(d_scratch)))
+    return fail(IE_B200_E_ARG, "ie_b200_attn_prefill: alignment");
+  if (T == 0) return IE_B200_OK;
+  if (n_head / n_kv > 8u) return fail(IE_B200_E_SIZE, "ie_b200_attn_prefill: %u query heads per KV head unsupported (1 .. 8)", n_head / n_kv);
   PtArgs a = {};
   a.q = d_q, a.out = d_out, a.oq = static_cast<uint8_t *>(d_oq), a.pos = d_pos;
   a.n_head = n_head, a.n_kv = n_kv, a.kv_len = kv_len, a.T = T, a.G = n_head / n_kv;
@@ -589,13 +596,6 @@ extern "C" size_t ie_b200_attn_prefill_scratch_bytes(uint32_t n_head, uint32_t h
 extern "C" int ie_b200_attn_prefill_split(const float *d_q, const void *d_kc, const void *d_vc, float *d_out, void *d_oq, const uint32_t *d_pos,
                                           uint32_t n_head, uint32_t n_kv, uint32_t hd, uint32_t kv_len, uint32_t T, size_t q_stride, size_t out_stride,
                                           size_t oq_stride, uint32_t positions, void *d_scratch, uint32_t *d_err, void *stream) {
-  if (!d_q || !d_kc || !d_vc || !d_out || !d_pos) return fail(IE_B200_E_ARG, "ie_b200_attn_prefill: NULL pointer");
-  if (n_kv == 0 || n_head % n_kv) return fail(IE_B200_E_SIZE, "ie_b200_attn_prefill: %u heads over %u KV heads", n_head, n_kv);
-  if (hd != 64 && hd != 128) return fail(IE_B200_E_SIZE, "ie_b200_attn_prefill: head dim %u (64, 128; half-precision cache)", hd);
-  if (!aligned16(d_kc) || !aligned16(d_vc) || ((uintptr_t)d_q & 7u) || (q_stride & 7u) || (d_scratch && !aligned16(d_scratch)))
-    return fail(IE_B200_E_ARG, "ie_b200_attn_prefill: alignment");
-  if (T == 0) return IE_B200_OK;
-  if (n_head / n_kv > 8u) return fail(IE_B200_E_SIZE, "ie_b200_attn_prefill: %u query heads per KV head unsupported (1 .. 8)", n_head / n_kv);
   return attn_prefill_tc(d_q, d_kc, d_vc, d_out, d_oq, d_pos, n_head, n_kv, hd, kv_len, T, q_stride, out_stride, oq_stride, positions,
                          static_cast<float *>(d_scratch), d_err, static_cast<cudaStream_t>(stream));
 }

@@ -9,6 +9,7 @@ namespace ieb {
 constexpr uint32_t PT_MAX_SPLITS = 16;
 // Scratch for the partial rows of up to PT_MAX_SPLITS splits of the positions.
 size_t attn_prefill_scratch_bytes(uint32_t n_head, uint32_t hd, uint32_t T);
+// The checks of the C entries are in here: the engine's call has them too.
 // positions: *d_pos + T as the host knows it (the grid is sized for it; the result does not depend on it). d_scratch NULL: one
 // split. d_err (may be NULL): set to 5 if a bounded wait inside the kernel ran out. hd 64 or 128.
 int attn_prefill_tc(const float *d_q, const void *d_kc, const void *d_vc, float *d_out, void *d_oq, const uint32_t *d_pos, uint32_t n_head, uint32_t n_kv,

@@ -245,6 +245,48 @@ def test_step_argument_checks(cuda):
     b.close()
 
 
+def test_chunk_attention_refuses_what_its_entry_refuses(cuda):
+    """An op list whose attention reads its queries 4 bytes off (offset or stride), or with more than 8 query heads per KV head:
+    refused on the host, as ie_b200_attn_prefill refuses it, and the engine goes on with a sound list."""
+    import ctypes as C
+
+    from amd_c_b200 import _lib
+    from amd_c_b200._lib import IeB200Error, Op, check
+    from amd_c_b200.backend import OP_ATTN
+
+    cfg = gguf.make_model(gguf.config("tiny-128"), seed=0)
+    b = Backend(cfg, 64, T=4)
+    want = b.run(0, [1, 2, 3], 0)
+
+    def with_attn(**kw):
+        arr = (Op * len(b.ops))(*b.ops)
+        for o in arr:
+            if o.kind == OP_ATTN:
+                for k, v in kw.items():
+                    setattr(o, k, getattr(o, k) + v)
+        check(b.lib.ie_b200_engine_set_ops(b.h, arr, len(b.ops), b.i_head))
+
+    for kw in ({"a": 4}, {"a_stride": 4}):
+        with_attn(**kw)
+        with pytest.raises(IeB200Error, match="alignment"):
+            b.run(0, [1, 2, 3], 0)
+    with_attn(a=0)
+    assert (b.run(0, [1, 2, 3], 0) == want).all()
+    b.close()
+    # nine query heads on one KV head: the attention op alone, on an engine without matrices
+    n = 9 * 64 * 4
+    d = _lib.EngineDesc(9, 1, 64, 64, 1, 4, 16, 1e-5, 0, 0, 8 * n + 64, 0, 8 * n, 64, 8)
+    h = C.c_void_p()
+    check(b.lib.ie_b200_engine_create(C.byref(d), C.byref(h)))
+    none = (1 << 64) - 1
+    ops = (Op * 1)(Op(OP_ATTN, -1, -1, 0, 9 * 64, 0, 0, 4 * n, none, none, none, n, n, 0, 0, 0))
+    check(b.lib.ie_b200_engine_set_ops(h, ops, 1, 1))
+    toks, out = np.array([1, 2], np.uint32), np.zeros(2, np.uint32)
+    with pytest.raises(IeB200Error, match="9 query heads"):
+        check(b.lib.ie_b200_engine_run(h, toks.ctypes.data_as(C.c_void_p), 2, 0, 1, out.ctypes.data_as(C.c_void_p), None))
+    b.lib.ie_b200_engine_destroy(h)
+
+
 @pytest.mark.parametrize("model", ["tiny", "tiny-k", "tiny-q8"])
 def test_ie_run_drop_in(cuda, tmp_path, model):
     """The reference's own ie-run host program (main.c, gen.c, model.c, plan.c compiled unchanged) linked with
