@@ -239,6 +239,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
           mx = fmaxf(fmaxf(mx, fmaxf(m4[0], m4[1])), fmaxf(m4[2], m4[3]));
         }
         mx *= a.scale_log2;
+        tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(pair);  // this warp has read all of S: the other may put P into it (waited for below, under the exponentials)
         if (j == 0) {
@@ -279,7 +280,10 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
             const __half2 lo = __floats2half2_rn(x, y);
             p[i] = *reinterpret_cast<const uint32_t *>(&h), p[16 + i] = *reinterpret_cast<const uint32_t *>(&lo);
           }
-          if (c == 0) ok = __all_sync(0xFFFFFFFFu, mbar_wait(pair, j & 1u, &s_abort));
+          if (c == 0) {
+            ok = __all_sync(0xFFFFFFFFu, mbar_wait(pair, j & 1u, &s_abort));
+            tc_fence_after();  // (the other warp's loads of S come before these stores, in tensor memory's order too)
+          }
           tc_st32(s_row + 32u * (2u * half + c), p);
         }
         {
