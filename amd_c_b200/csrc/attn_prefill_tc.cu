@@ -17,7 +17,9 @@
 // Shared memory: Q as MMA core matrices (hd x 256 B per term and tile), a ring of three K or V blocks (128 rows) brought by
 // TMA in the 128-byte swizzle (boxes of 64 columns), one thread issuing. (cp.async in 16-byte pieces needed some 3500 cycles
 // to issue a block from three warps and left the tensor pipe half idle.) V rows past the last position are zeroed in shared
-// memory after they have landed: the cache may hold anything there, and 0 x NaN is not 0.
+// memory after they have landed: the cache may hold anything there, and 0 x NaN is not 0. For the same reason the blocks that
+// some row of the CTA does not see whole are looked through for infinities and NaN (a value that overflowed the half cache must
+// not reach the tokens before it): they are replaced by zeros, and added at the end to the rows that do see them.
 // O is rescaled lazily: only when a row's maximum has grown by more than 2^8 (p stays far inside f16).
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -44,6 +46,7 @@ struct PtArgs {
   uint32_t wide;     // bit 0: the rows written are 16-byte aligned, bit 1: the q rows are
   uint32_t tiles;    // 128-row tiles per CTA: 1 or 2
   float inv_g;       // 1 / G
+  const __half *vc;  // the V cache (read here only for rows that hold an infinity or a NaN)
 };
 
 __device__ __forceinline__ float ex2(float x) {
@@ -101,6 +104,12 @@ __device__ __forceinline__ void store_row4(float *out, size_t out_stride, uint8_
   if ((at & 31u) == 0u) reinterpret_cast<float *>(qrow + 32u * (size_t)nbq)[at / 32u] = d, reinterpret_cast<int *>(qrow + 36u * (size_t)nbq)[at / 32u] = sum;
 }
 
+__device__ __forceinline__ __half2 as_half2(uint32_t w) { return *reinterpret_cast<const __half2 *>(&w); }
+// Two halves in a word: all ones in the place of each that is an infinity or a NaN.
+__device__ __forceinline__ uint32_t half_bad(uint32_t w) {
+  return ((w & 0x7C00u) == 0x7C00u ? 0xFFFFu : 0u) | ((w & 0x7C000000u) == 0x7C000000u ? 0xFFFF0000u : 0u);
+}
+
 // r / G for r below 2^22 (exact: r + 0.5 is at least 0.5 / G away from a multiple of G, the product's error below 2^-23 of it)
 __device__ __forceinline__ uint32_t row_token(uint32_t r, float inv_g) { return (uint32_t)(((float)r + 0.5f) * inv_g); }
 
@@ -118,14 +127,14 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
   uint64_t *kv_full = bars, *kv_empty = bars + PT_RING, *s_full = bars + 2 * PT_RING, *p_full = s_full + 2, *q_full = p_full + 2, *drained = q_full + 1,
            *tail = drained + 1, *pair_bar = tail + 1;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(pair_bar + 8);
-  volatile uint32_t &s_abort = *(tmem_slot + 1);
+  volatile uint32_t &s_abort = *(tmem_slot + 1), &s_bad = *(tmem_slot + 2);  // s_bad: zeros stand for infinities or NaN in V
   float *s_pair = reinterpret_cast<float *>(smem_pt + L::PAIR_OFF);  // [tile][half][row]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t g = blockIdx.y, split = blockIdx.z, rows_total = a.T * a.G, row0 = blockIdx.x * 128u * a.tiles;
   const uint32_t n_tiles = a.tiles == 2u && rows_total - row0 > 128u ? 2u : 1u;
 
   if (threadIdx.x == 0) {
-    s_abort = 0u;
+    s_abort = 0u, s_bad = 0u;
     for (int i = 0; i < PT_RING; i++) mbar_init(&kv_full[i], 1u), mbar_init(&kv_empty[i], 1u);
     for (int t = 0; t < 2; t++) mbar_init(&s_full[t], 1u), mbar_init(&p_full[t], 8u);
     mbar_init(q_full, 8u * n_tiles), mbar_init(drained, 1u), mbar_init(tail, 1u);
@@ -206,6 +215,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
       }
       positions();
       const uint32_t lim = real ? pos0 + tok + 1u : 0xFFFFFFFFu;  // positions this row sees (rows past the last are never stored)
+      const uint32_t first_lim = pos0 + row_token(row0, a.inv_g) + 1u;  // the fewest that a row of the CTA sees
       float m = -INFINITY, l = 0.0f;  // maximum the row's terms are taken against (log2 units), sum of this thread's terms
       bool ok = true;
       for (uint32_t j = 0; j < n; j++) {
@@ -291,6 +301,30 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
           f32x2_parts(sum2, x, y);
           l += x + y;
         }
+        if (t == 0u && k0 + PT_KEYS > first_lim) {  // the first tile's warps, ahead of every product with this block of V
+          const uint32_t u = 2u * j + 1u;
+          ok = ok && __all_sync(0xFFFFFFFFu, mbar_wait(&kv_full[u % PT_RING], (u / PT_RING) & 1u, &s_abort));
+          if (ok) {
+            uint4 *vb = reinterpret_cast<uint4 *>(smem_pt + L::KV_OFF + (u % PT_RING) * L::BLOCK) + threadIdx.x;
+            __half2 top = __float2half2_rn(0.0f);
+#pragma unroll
+            for (int i = 0; i < (int)(L::BLOCK / 4096u); i++) {
+              const uint4 x = vb[i * 256];
+              top = __hmax2_nan(__hmax2_nan(top, __habs2(as_half2(x.x))), __habs2(as_half2(x.y)));
+              top = __hmax2_nan(__hmax2_nan(top, __habs2(as_half2(x.z))), __habs2(as_half2(x.w)));
+            }
+            if (half_bad(*reinterpret_cast<const uint32_t *>(&top))) {
+#pragma unroll 1
+              for (int i = 0; i < (int)(L::BLOCK / 4096u); i++) {
+                uint4 x = vb[i * 256];
+                x.x &= ~half_bad(x.x), x.y &= ~half_bad(x.y), x.z &= ~half_bad(x.z), x.w &= ~half_bad(x.w);
+                vb[i * 256] = x;
+              }
+              s_bad = 1u;
+              fence_async_shared();
+            }
+          }
+        }
         if (!ok) break;
         tc_wait_st();
         tc_fence_before();
@@ -324,6 +358,21 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
           uint32_t v[32];
           tc_ld32(o_col + 32u * c, v);
           tc_wait_ld();
+          if (s_bad && real) {  // what the zeros in V stand for, for the positions that this row sees (every such p is positive)
+            const uint32_t k1 = min(lim, (b0 + n) * PT_KEYS);
+#pragma unroll 1
+            for (uint32_t k = max(b0 * PT_KEYS, first_lim / PT_KEYS * PT_KEYS); k < k1; k++) {
+              const uint32_t *vr = reinterpret_cast<const uint32_t *>(a.vc + ((size_t)g * a.kv_len + k) * HD + half * (HD / 2u) + 32u * c);
+#pragma unroll
+              for (int i = 0; i < 16; i++) {
+                const uint32_t w = vr[i], bad = half_bad(w);
+                if (bad) {
+                  const float2 f = __half22float2(as_half2(w & bad));  // (0 where the half is finite)
+                  v[2 * i] = __float_as_uint(__uint_as_float(v[2 * i]) + f.x), v[2 * i + 1] = __float_as_uint(__uint_as_float(v[2 * i + 1]) + f.y);
+                }
+              }
+            }
+          }
 #pragma unroll
           for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * inv);
 #pragma unroll
@@ -581,6 +630,7 @@ int attn_prefill_tc(const float *d_q, const void *d_kc, const void *d_vc, float 
   a.q_stride = q_stride, a.out_stride = out_stride, a.oq_stride = oq_stride;
   a.scale_log2 = 1.44269504088896340736f / sqrtf((float)hd);
   a.err = d_err;
+  a.vc = static_cast<const __half *>(d_vc);
   uint32_t splits = 1u, tiles = 1u;
   a.wide = ((((uintptr_t)d_out | out_stride) & 15u) == 0u ? 1u : 0u) | ((((uintptr_t)d_q | q_stride) & 15u) == 0u ? 2u : 0u);
   a.inv_g = 1.0f / (float)a.G;

@@ -793,6 +793,44 @@ def test_attention_prefill_empty_splits(cuda, lib, n_head, n_kv, hd, T, pos0):
     assert int(err.item()) == 0
 
 
+@pytest.mark.parametrize("n_head,n_kv,hd,T,pos0", [(8, 8, 64, 256, 100), (28, 4, 128, 64, 1000), (8, 2, 128, 70, 58), (3, 1, 64, 17, 0)])
+@pytest.mark.parametrize("split", [False, True])
+def test_attention_prefill_infinite_values(cuda, n_head, n_kv, hd, T, pos0, split):
+    """A V value that overflowed the half cache (or a NaN) belongs to the tokens that see its position: the rows of the tokens
+    before it, and the other columns of the rows behind it, are bit for bit those of the run with finite values."""
+    import torch
+
+    from amd_c_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    n, G = pos0 + T, n_head // n_kv
+    kc, vc = (torch.randn((n_kv, n, hd), generator=gen, device=cuda).half() for _ in range(2))
+    q = torch.randn((T, n_head * hd), generator=gen, device=cuda)
+    pos = torch.tensor([pos0], dtype=torch.int32, device=cuda)
+
+    def run(v):
+        if not split:
+            return K.attn_prefill(q, kc, v, pos, n_head, n_kv, hd)
+        out, oq, err = K.attn_prefill_split(q, kc, v, pos, n_head, n_kv, hd, n)
+        assert int(err.item()) == 0
+        return out, oq
+
+    want, _ = run(vc)
+    assert torch.isfinite(want).all()
+    bad = {(0, T - 1, 5): float("inf"), (n_kv - 1, T // 2, hd - 1): -float("inf"), (n_kv - 1, T // 2 + 1, hd // 2): float("nan"), (0, 1, 33): float("inf")}
+    v = vc.clone()
+    hit = torch.zeros((T, n_kv, G, hd), dtype=torch.bool, device=cuda)
+    for (g, t, d), x in bad.items():
+        v[g, pos0 + t, d] = x
+        hit[t:, g, :, d] = True
+    got, oq = run(v)
+    hit = hit.view(T, n_head * hd)
+    assert torch.equal(got[~hit].view(torch.int32), want[~hit].view(torch.int32))
+    assert not torch.isfinite(got[hit]).any()
+    rows = ~hit.any(1)
+    assert torch.equal(oq[rows], K.quant_q8(got[rows]))
+
+
 @pytest.mark.parametrize("typ,rows,cols,T", [(synth.GGML_Q4_0, 130, 1024, 11), (synth.GGML_Q4_K, 77, 512, 16), (synth.GGML_Q6_K, 40, 18944, 5),
                                              (synth.GGML_Q4_0, 9, 64, 2), (synth.GGML_Q8_0, 130, 1024, 11), (synth.GGML_Q8_0, 40, 4096, 16)])
 def test_gemv_several_tokens_one_pass(ora, cuda, typ, rows, cols, T):
