@@ -152,14 +152,18 @@ static bool tc_gemm(const ie_b200_engine *e, const ie_b200_op &o, uint32_t T) {
   return o.kind == IE_B200_OP_GEMV && o.mat >= 0 && (size_t)o.mat < e->mats.size() && T >= 17 && e->mats[o.mat].kind != IE_B200_MAT_F32 && !e->no_gemm &&
          !e->gemm_mma && o.a_stride % 16u == 0 && !few_tokens(e->mats[o.mat], T);
 }
+// Do T rows of an bytes at a and T rows of bn bytes at b have no byte in common? (Says no where rows of different strides interleave.)
+static bool rows_apart(uint64_t a, uint32_t as, uint64_t an, uint64_t b, uint32_t bs, uint64_t bn, uint32_t T) {
+  const uint64_t last = T - 1u;  // in 64 bits: a stride times the tokens may pass 4 GB
+  if (b >= a + as * last + an || a >= b + bs * last + bn) return true;
+  return as == bs && ((a + an <= b && b + bn <= a + as) || (b + bn <= a && a + an <= b + bs));
+}
 // Are the expanded activations that GEMM op p left in the scratch also those of op o, launched right after it with nothing
 // between them (q, k and v of a layer)? The same Q8 rows, and p's result does not lie over them: all of it before or behind
 // them, or, token rows interleaved, beside them in every row.
 static bool tc_same_act(const ie_b200_engine *e, const ie_b200_op &p, const ie_b200_op &o, uint32_t T) {
   if (!tc_gemm(e, p, T) || !tc_gemm(e, o, T) || p.a != o.a || p.a_stride != o.a_stride || e->mats[p.mat].cols != e->mats[o.mat].cols) return false;
-  const uint64_t an = e->mats[p.mat].cols / 32u * 40ull, bn = 4ull * e->mats[p.mat].rows;
-  if (p.b >= p.a + p.a_stride * (T - 1u) + an || p.a >= p.b + p.b_stride * (T - 1u) + bn) return true;
-  return p.a_stride == p.b_stride && ((p.a + an <= p.b && p.b + bn <= p.a + p.a_stride) || (p.b + bn <= p.a && p.a + an <= p.b + p.b_stride));
+  return rows_apart(p.a, p.a_stride, e->mats[p.mat].cols / 32u * 40ull, p.b, p.b_stride, 4ull * e->mats[p.mat].rows, T);
 }
 
 // One op for tokens [t0, t0 + T) of a run. prev: the op launched right before it for the same tokens, or NULL.

@@ -1,0 +1,98 @@
+"""The engine below the model: op lists of a few GEMVs over hand-made rows."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from amd_c_b200 import synth
+
+pytestmark = pytest.mark.gpu
+NONE = (1 << 64) - 1
+
+
+class Engine:
+    """An engine with its own arena and matrices, run on op lists given as (matrix, offset of the Q8 rows, stride, offset of the
+    result, stride)."""
+
+    def __init__(self, arena_bytes: int, T: int):
+        from amd_c_b200 import _lib
+
+        self.lib, self.T, self.arena = _lib.load(), T, arena_bytes
+        self.h, self.keep = C.c_void_p(), []
+        d = _lib.EngineDesc(1, 1, 64, 64, 1, T, 16, 1e-5, 0, 0, arena_bytes + 64 * T, arena_bytes, arena_bytes, 64, 8)
+        self.check(self.lib.ie_b200_engine_create(C.byref(d), C.byref(self.h)))
+
+    def check(self, r):
+        from amd_c_b200._lib import check
+
+        check(r)
+
+    def add(self, m) -> int:
+        self.keep.append(m)
+        return self.lib.ie_b200_engine_add_mat_device(self.h, m.kind, m.rows, m.cols, m.data.data_ptr())
+
+    def write(self, off: int, row: np.ndarray):
+        row = np.ascontiguousarray(row)
+        self.check(self.lib.ie_b200_engine_write_rows(self.h, off, row.nbytes, 0, 1, row.ctypes.data_as(C.c_void_p)))
+
+    def read(self, off: int, n: int) -> np.ndarray:
+        out = np.zeros(n, np.float32)
+        self.check(self.lib.ie_b200_engine_read_rows(self.h, off, 4 * n, 0, 1, out.ctypes.data_as(C.c_void_p)))
+        return out
+
+    def run(self, gemvs):
+        from amd_c_b200._lib import Op
+        from amd_c_b200.backend import OP_GEMV
+
+        ops = [Op(OP_GEMV, m, -1, -1, 0, 0, a, b, NONE, NONE, NONE, a_s, b_s, 0, 0, 0) for m, a, a_s, b, b_s in gemvs]
+        self.check(self.lib.ie_b200_engine_set_ops(self.h, (Op * len(ops))(*ops), len(ops), len(ops)))
+        toks, out = np.zeros(self.T, np.uint32), np.zeros(self.T, np.uint32)
+        self.check(self.lib.ie_b200_engine_run(self.h, toks.ctypes.data_as(C.c_void_p), self.T, 0, 1, out.ctypes.data_as(C.c_void_p), None))
+
+    def close(self):
+        self.lib.ie_b200_engine_destroy(self.h)
+
+
+def _q8(torch, K, rng, T, cols, cuda):
+    return K.quant_q8(torch.from_numpy(rng.standard_normal((T, cols)).astype(np.float32)).to(cuda)).cpu().numpy()
+
+
+def test_expanded_activations_are_shared_only_where_they_still_hold(cuda):
+    """GEMMs over the same Q8 rows, one after the other, share the expanded activations: bit for bit what each gives in a run of its
+    own. Not where another GEMM's rows come between, and not where the first one's result lies over the Q8 rows, here with token
+    rows 256 MB apart, so that the extent of 26 of them (6.7 GB) does not fit 32 bits."""
+    import torch
+
+    from amd_c_b200 import kernels as K
+
+    rng = np.random.default_rng(8)
+    T, cols, rows, S = 26, 4096, 16, 1 << 28
+    e = Engine(26 * S, T)
+    mats = [e.add(K.Mat.from_gguf(t, torch.from_numpy(np.ascontiguousarray(synth.make_gguf_bytes(t, rng, rows, cols))).to(cuda), rows, cols))
+            for t in (synth.GGML_Q4_K, synth.GGML_Q4_K, synth.GGML_Q6_K)]
+    x, z = _q8(torch, K, rng, T, cols, cuda), _q8(torch, K, rng, T, cols, cuda)
+    zoff = 1 << 20  # of the other rows, behind the first ones of the same token
+
+    def fill():
+        for t in range(T):
+            e.write(S * t, x[t]), e.write(S * t + zoff, z[t])
+
+    def results(ops):
+        return [np.stack([e.read(b + bs * t, rows) for t in range(T)]).view(np.uint32) for _, _, _, b, bs in ops]
+
+    beside = [(mats[i], 0, S, (2 << 20) + 4096 * i, S) for i in range(3)]          # q, k and v of a layer
+    between = [beside[0], (mats[1], zoff, S, beside[1][3], S), beside[2]]           # other rows come between
+    # the first result's rows lie back to back over the bytes of token 10's Q8 row (values only: its scales stay)
+    over = [(mats[0], 0, S, 10 * S, 4 * rows), (mats[1], 0, S, 2 << 20, S), (mats[2], 0, S, (2 << 20) + 4096, S)]
+    assert T * 4 * rows <= cols
+    for ops in (beside, between, over):
+        fill()
+        e.run(ops)
+        got = results(ops)
+        fill()
+        for op in ops:
+            e.run([op])
+        want = results(ops)
+        for g, w in zip(got, want):
+            assert (g == w).all()
+    e.close()
