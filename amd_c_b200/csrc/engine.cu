@@ -147,7 +147,8 @@ static bool stream_ok(const EMat &m) { return gemv_direct_ok(m.kind, m.cols); }
 // Q6_K, two tensor products per block (2048 x 4096 15 .. 16 / 15); at 28 tokens it is level (66 / 71, 20 / 19, 83 / 77).
 static bool few_tokens(const EMat &m, uint32_t T) { return T <= 24u && m.cols <= 6144u && m.kind != IE_B200_MAT_Q6K; }
 
-// Does the tcgen05 GEMM run op o over T tokens? (From the reference's threshold on, src/hip.c:965.)
+// Does the tcgen05 GEMM run op o over T tokens? (From the reference's threshold on, src/hip.c:965.) The one place that says so:
+// launch_op dispatches by it, and tc_same_act relies on it to know what the scratch holds.
 static bool tc_gemm(const ie_b200_engine *e, const ie_b200_op &o, uint32_t T) {
   return o.kind == IE_B200_OP_GEMV && o.mat >= 0 && (size_t)o.mat < e->mats.size() && T >= 17 && e->mats[o.mat].kind != IE_B200_MAT_F32 && !e->no_gemm &&
          !e->gemm_mma && o.a_stride % 16u == 0 && !few_tokens(e->mats[o.mat], T);
@@ -195,29 +196,28 @@ static int launch_op(ie_b200_engine *e, const ie_b200_op &o, uint32_t t0, uint32
       const float *bias = o.vec >= 0 ? e->vecs[o.vec].d : nullptr;
       if (T == 1 && stream_ok(m))
         return ie_b200_gemv_stream(m.kind, m.d, m.rows, m.cols, a, static_cast<float *>(b), bias, static_cast<float *>(res), st);
-      // a prompt chunk (the reference's threshold, src/hip.c:965): the tensor-core GEMM reads the weights once per 128 tokens
-      const bool tc_ok = !e->gemm_mma && o.a_stride % 16u == 0;
-      // (Q8_0 has no mma.sync form: where the tcgen05 kernel cannot run it takes the multi-token GEMV below, 8 tokens per pass)
-      if (T >= 17 && m.kind != IE_B200_MAT_F32 && !e->no_gemm && (tc_ok || m.kind != IE_B200_MAT_Q8) && !(tc_ok && few_tokens(m, T))) {
-        if (tc_ok) {  // tcgen05 / tensor memory
-          EMat &mm = e->mats[o.mat];
-          // (normally done by prepare_chunks before anything of the run is enqueued; here for callers that enqueue ranges themselves)
-          if (mm.tc_exp == INT32_MIN)
-            if (int r = ie_b200_mat_tc_exp(mm.kind, mm.d, mm.rows, mm.cols, &mm.tc_exp, st)) return r;
-          const size_t need = ie_b200_gemm_tc_scratch_bytes(mm.rows, mm.cols, e->d.T_max);
-          if (need > e->gemm_scratch_bytes) {
-            IEB_CUDA(cudaStreamSynchronize(st));
-            cudaFree(e->gemm_scratch), e->gemm_scratch = nullptr, e->gemm_scratch_bytes = 0;
-            IEB_CUDA(cudaMalloc(&e->gemm_scratch, need));
-            e->gemm_scratch_bytes = need;
-            prev = nullptr;
-          }
-          return gemm_tc_run(mm.kind, mm.d, mm.rows, mm.cols, mm.tc_exp, a, static_cast<float *>(b), bias, static_cast<float *>(res), T, o.a_stride, o.b_stride,
-                             o.res_stride, e->gemm_scratch, e->gemm_scratch_bytes, e->err, st, prev && tc_same_act(e, *prev, o, T));
+      // a prompt chunk: the tensor-core GEMM reads the weights once per 256 tokens
+      if (tc_gemm(e, o, T)) {  // tcgen05 / tensor memory
+        EMat &mm = e->mats[o.mat];
+        // (normally done by prepare_chunks before anything of the run is enqueued; here for callers that enqueue ranges themselves)
+        if (mm.tc_exp == INT32_MIN)
+          if (int r = ie_b200_mat_tc_exp(mm.kind, mm.d, mm.rows, mm.cols, &mm.tc_exp, st)) return r;
+        const size_t need = ie_b200_gemm_tc_scratch_bytes(mm.rows, mm.cols, e->d.T_max);
+        if (need > e->gemm_scratch_bytes) {
+          IEB_CUDA(cudaStreamSynchronize(st));
+          cudaFree(e->gemm_scratch), e->gemm_scratch = nullptr, e->gemm_scratch_bytes = 0;
+          IEB_CUDA(cudaMalloc(&e->gemm_scratch, need));
+          e->gemm_scratch_bytes = need;
+          prev = nullptr;
         }
+        return gemm_tc_run(mm.kind, mm.d, mm.rows, mm.cols, mm.tc_exp, a, static_cast<float *>(b), bias, static_cast<float *>(res), T, o.a_stride, o.b_stride,
+                           o.res_stride, e->gemm_scratch, e->gemm_scratch_bytes, e->err, st, prev && tc_same_act(e, *prev, o, T));
+      }
+      // the mma.sync form where it is asked for, or the Q8 rows are not 16-byte aligned. (It has no Q8_0 form: that takes the
+      // multi-token GEMV below, as do a few tokens: up to 16 tokens per pass over the weights.)
+      if (T >= 17 && m.kind != IE_B200_MAT_F32 && m.kind != IE_B200_MAT_Q8 && !e->no_gemm && (e->gemm_mma || o.a_stride % 16u != 0))
         return ie_b200_gemm(m.kind, m.d, m.rows, m.cols, a, static_cast<float *>(b), bias, static_cast<float *>(res), T, o.a_stride, o.b_stride,
                             o.res_stride, st);
-      }
       return ie_b200_gemv(m.kind, m.d, m.rows, m.cols, a, static_cast<float *>(b), bias, static_cast<float *>(res), T, o.a_stride, o.b_stride,
                           o.res_stride, st);
     }
