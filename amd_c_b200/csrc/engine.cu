@@ -85,7 +85,6 @@ struct ie_b200_engine {
   void *topk_scratch = nullptr;  // candidates and results of ie_b200_engine_topk
   size_t topk_bytes = 0;
   float *pf_scratch = nullptr;   // the prompt-chunk attention's partial rows
-  uint32_t run_hi = 0;           // positions that the chunk begun last reaches (0: unknown, ops enqueued by the caller)
   void *gemm_scratch = nullptr;  // expanded activations and K-split partials of the tcgen05 GEMM
   size_t gemm_scratch_bytes = 0;
   int norm_mode = 2;         // IE_B200_NORM: 2 (default) a kernel of its own, 0 "tail": in the producing GEMV's last CTA, 1 "prologue": in the consuming GEMVs
@@ -167,8 +166,9 @@ static bool tc_same_act(const ie_b200_engine *e, const ie_b200_op &p, const ie_b
   return rows_apart(p.a, p.a_stride, e->mats[p.mat].cols / 32u * 40ull, p.b, p.b_stride, 4ull * e->mats[p.mat].rows, T);
 }
 
-// One op for tokens [t0, t0 + T) of a run. prev: the op launched right before it for the same tokens, or NULL.
-static int launch_op(ie_b200_engine *e, const ie_b200_op &o, uint32_t t0, uint32_t T, cudaStream_t st, const ie_b200_op *prev = nullptr) {
+// One op for tokens [t0, t0 + T) of a run. prev: the op launched right before it for the same tokens, or NULL. hi: positions that
+// the tokens reach, as the host knows it (it sizes the chunk attention's grid), or 0: ops enqueued by the caller.
+static int launch_op(ie_b200_engine *e, const ie_b200_op &o, uint32_t t0, uint32_t T, cudaStream_t st, const ie_b200_op *prev = nullptr, uint32_t hi = 0) {
   const ie_b200_engine_desc &d = e->d;
   void *a = at(e, o.a, o.a_stride, t0), *b = at(e, o.b, o.b_stride, t0), *c = at(e, o.c, o.c_stride, t0);
   void *qo = at(e, o.qo, o.qo_stride, t0), *res = at(e, o.res, o.res_stride, t0);
@@ -234,7 +234,7 @@ static int launch_op(ie_b200_engine *e, const ie_b200_op &o, uint32_t t0, uint32
       if (T > 1 && !d.kv_f32 && (d.hd == 64 || d.hd == 128) && !e->no_prefill_attn)
         return attn_prefill_tc(static_cast<float *>(at(e, o.a, o.a_stride, t0)), kcl, vcl, static_cast<float *>(at(e, o.b, o.b_stride, t0)),
                                at(e, o.qo, o.qo_stride, t0), pos + 1 + t0, d.n_head, d.n_kv, d.hd, d.n_ctx, T, o.a_stride, o.b_stride, o.qo_stride,
-                               e->run_hi, e->run_hi ? e->pf_scratch : nullptr, e->err, st);
+                               hi, hi ? e->pf_scratch : nullptr, e->err, st);
       for (uint32_t s = 0; s < T; s += e->T_att) {  // bounded scratch: at most T_att tokens per launch
         const uint32_t n = T - s < e->T_att ? T - s : e->T_att;
         int r = ie_b200_attn_decode(static_cast<float *>(at(e, o.a, o.a_stride, t0 + s)), kcl, vcl, static_cast<float *>(at(e, o.b, o.b_stride, t0 + s)),
@@ -1059,12 +1059,10 @@ extern "C" int ie_b200_engine_run_begin(ie_b200_engine *e, const uint32_t *toks,
   cudaStream_t st = e->stream;
   if (int r = upload_input(e, toks, T, pos, st)) return r;
   const uint32_t n_ops = (uint32_t)e->ops.size(), ih = last_only ? e->i_head : n_ops;
-  e->run_hi = pos + T;
   for (uint32_t i = 0; i < ih; i++)
-    if (int r = launch_op(e, e->ops[i], 0, T, st, i ? &e->ops[i - 1] : nullptr)) return r;
+    if (int r = launch_op(e, e->ops[i], 0, T, st, i ? &e->ops[i - 1] : nullptr, pos + T)) return r;
   for (uint32_t i = ih; i < n_ops; i++)  // the output head for the last token only
     if (int r = launch_op(e, e->ops[i], T - 1, 1, st)) return r;
-  e->run_hi = 0;
   IEB_CUDA(cudaMemcpy2DAsync(e->h_result, 8, e->arena + e->d.argmax_off, e->d.argmax_stride ? e->d.argmax_stride : 8, 8, T, cudaMemcpyDeviceToHost, st));
   IEB_CUDA(cudaMemcpyAsync(e->h_result + 2 * e->d.T_max, e->err, 4, cudaMemcpyDeviceToHost, st));
   e->run_T = T;
