@@ -25,6 +25,8 @@
 #include <cudaTypedefs.h>
 #include <math.h>
 
+#include <algorithm>
+
 #include "attn_prefill_tc.cuh"
 #include "tc_common.cuh"
 
@@ -587,7 +589,7 @@ static void pick_shape(uint32_t rows, uint32_t n_kv, uint32_t blocks, uint32_t a
   float best = 1e30f;
   for (uint32_t t = 1; t <= 2u; t++) {
     const uint32_t ctas = (rows + 128u * t - 1u) / (128u * t) * n_kv;
-    for (uint32_t s = 1; s <= (may_split ? PT_MAX_SPLITS : 1u) && s <= blocks; s++) {
+    for (uint32_t s = 1; s <= (may_split ? PT_MAX_SPLITS : 1u) && s <= blocks && (s == 1u || s * all_rows <= PT_MAX_RECORDS); s++) {
       const uint32_t per = (blocks + s - 1u) / s, waves = (ctas * s + sms - 1u) / sms;
       float cost = (float)waves * (t == 2u ? (float)per * 3.5f + 8.0f : (float)per * 2.9f + 5.0f);
       if (s > 1u) cost += 3.5f + (float)s * (float)all_rows * (float)hd * 8.0f / 4.0e6f;
@@ -597,7 +599,7 @@ static void pick_shape(uint32_t rows, uint32_t n_kv, uint32_t blocks, uint32_t a
 }
 
 size_t attn_prefill_scratch_bytes(uint32_t n_head, uint32_t hd, uint32_t T) {
-  return (size_t)PT_MAX_SPLITS * T * n_head * (hd + 2u) * sizeof(float) + 256u;
+  return std::min((size_t)PT_MAX_SPLITS * T * n_head, (size_t)PT_MAX_RECORDS) * (hd + 2u) * sizeof(float) + 256u;
 }
 
 template <int HD>

@@ -6,8 +6,10 @@
 
 namespace ieb {
 
-constexpr uint32_t PT_MAX_SPLITS = 16;
-// Scratch for the partial rows of up to PT_MAX_SPLITS splits of the positions.
+// Splits of the positions, and partial rows of all of them together, at most. (16 splits of 256 tokens x 80 heads: a chunk with
+// more rows fills the GPU with fewer splits. The scratch stays below 171 MB, heads of 128, however long the chunks.)
+constexpr uint32_t PT_MAX_SPLITS = 16, PT_MAX_RECORDS = 16u * 256u * 80u;
+// Scratch for the partial rows.
 size_t attn_prefill_scratch_bytes(uint32_t n_head, uint32_t hd, uint32_t T);
 // The checks of the C entries are in here: the engine's call has them too.
 // positions: *d_pos + T as the host knows it (the grid is sized for it; the result does not depend on it). d_scratch NULL: one

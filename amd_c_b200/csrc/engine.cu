@@ -84,7 +84,7 @@ struct ie_b200_engine {
                              // the whole vector itself, which costs more than the launch it saves (measured at 1 and 2 GPUs)
   void *topk_scratch = nullptr;  // candidates and results of ie_b200_engine_topk
   size_t topk_bytes = 0;
-  float *pf_scratch = nullptr;   // the prompt-chunk attention's partial rows
+  float *pf_scratch = nullptr;   // the prompt-chunk attention's partial rows (NULL: it walks the positions in one split)
   void *gemm_scratch = nullptr;  // expanded activations and K-split partials of the tcgen05 GEMM
   size_t gemm_scratch_bytes = 0;
   int norm_mode = 2;         // IE_B200_NORM: 2 (default) a kernel of its own, 0 "tail": in the producing GEMV's last CTA, 1 "prologue": in the consuming GEMVs
@@ -1029,8 +1029,9 @@ extern "C" int ie_b200_engine_enqueue_kinds(ie_b200_engine *e, uint32_t first, u
 // once per engine (the scratch), made ready BEFORE anything of the run is enqueued: both wait for the stream, and a wait in
 // the middle of a run would wait for exchange kernels whose partners on other GPUs this thread has not enqueued yet.
 static int prepare_chunks(ie_b200_engine *e, uint32_t T) {
-  if (T > 1 && !e->pf_scratch && !e->d.kv_f32 && (e->d.hd == 64 || e->d.hd == 128) && !e->no_prefill_attn)
-    IEB_CUDA(cudaMalloc(&e->pf_scratch, attn_prefill_scratch_bytes(e->d.n_head, e->d.hd, e->d.T_max)));
+  if (T > 1 && !e->pf_scratch && !e->d.kv_f32 && (e->d.hd == 64 || e->d.hd == 128) && !e->no_prefill_attn &&
+      cudaMalloc(&e->pf_scratch, attn_prefill_scratch_bytes(e->d.n_head, e->d.hd, e->d.T_max)) != cudaSuccess)
+    e->pf_scratch = nullptr, cudaGetLastError();  // no room: slower, not refused
   if (T < 17 || e->no_gemm || e->gemm_mma) return IE_B200_OK;
   size_t need = 0;
   for (const ie_b200_op &o : e->ops) {

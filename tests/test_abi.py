@@ -42,3 +42,14 @@ def test_bad_arguments_are_refused(lib):
     assert lib.ie_b200_gemv(99, p, 8, 64, p, p, None, None, 1, 0, 0, 0, None) == -1
     assert lib.ie_b200_gemv(_lib.MAT_Q4K, p, 8, 64, p, p, None, None, 1, 0, 0, 0, None) == -2  # K kinds need cols % 256 == 0
     assert lib.ie_b200_attn_decode(p, p, p, p, None, p, 8, 3, 32, 0, 64, 64, 1, 0, 0, 0, p, p, None) == -2  # 8 heads over 3 KV heads
+
+
+def test_attention_chunk_scratch_is_bounded(lib):
+    """Scratch of the chunk attention: 16 splits of a chunk of 256 tokens, and no more than 171 MB however long the chunks are."""
+    size = lib.ie_b200_attn_prefill_scratch_bytes
+    assert size(40, 128, 256) == 16 * 256 * 40 * 130 * 4 + 256
+    assert size(40, 128, 2048) == size(40, 128, 8192) == 16 * 256 * 80 * 130 * 4 + 256
+    for heads in (1, 8, 28, 40, 64):
+        for hd in (64, 128):
+            sizes = [size(heads, hd, T) for T in (1, 2, 17, 77, 256, 300, 2048, 8192)]
+            assert sizes == sorted(sizes) and sizes[-1] <= 171 << 20

@@ -96,3 +96,52 @@ def test_expanded_activations_are_shared_only_where_they_still_hold(cuda):
         for g, w in zip(got, want):
             assert (g == w).all()
     e.close()
+
+
+def test_chunk_without_room_for_the_attention_scratch(cuda):
+    """Where the chunk attention's scratch (85 MB here) cannot be had, the chunk runs with one split of the positions: the same rows
+    to the summation order, not an error. (One accumulator takes 16 products per 128 positions, 256 for these, and loses up to one
+    unit of 24 bits with each: 1.6e-5 of the scale.)"""
+    import torch
+
+    from amd_c_b200 import _lib
+    from amd_c_b200._lib import Op, check
+    from amd_c_b200.backend import OP_ATTN, OP_ROPE_KV
+
+    lib = _lib.load()
+    nh, nkv, hd, T, n_ctx = 40, 8, 128, 256, 2048
+    row, orow = (nh + 2 * nkv) * hd * 4, nh * hd * 4
+    ops = (Op * 2)(Op(OP_ROPE_KV, -1, -1, 0, nh * hd, nh, 0, nh * hd * 4, (nh + nkv) * hd * 4, NONE, NONE, row, row, row, 0, 0),
+                   Op(OP_ATTN, -1, -1, 0, nh * hd, 0, 0, T * row, NONE, NONE, NONE, row, orow, 0, 0, 0))
+    d = _lib.EngineDesc(nh, nkv, hd, n_ctx, 1, T, 16, 1e-5, 0, 0, T * (row + orow) + 64 * T, T * (row + orow), T * (row + orow), 64, 8)
+    one, zero = np.ones((n_ctx, hd // 2), np.float32), np.zeros((n_ctx, hd // 2), np.float32)
+    engines = []
+    for _ in range(2):
+        h = C.c_void_p()
+        check(lib.ie_b200_engine_create(C.byref(d), C.byref(h)))
+        check(lib.ie_b200_engine_set_rope(h, one.ctypes.data_as(C.c_void_p), zero.ctypes.data_as(C.c_void_p)))
+        check(lib.ie_b200_engine_set_ops(h, ops, 2, 2))
+        engines.append(h)
+    toks, out = np.zeros(T, np.uint32), np.zeros(T, np.uint32)
+
+    def chunks(h):
+        rng = np.random.default_rng(2)
+        for pos in range(0, n_ctx, T):
+            x = rng.standard_normal((T, row // 4)).astype(np.float32)
+            check(lib.ie_b200_engine_write_rows(h, 0, row, 0, T, x.ctypes.data_as(C.c_void_p)))
+            check(lib.ie_b200_engine_run(h, toks.ctypes.data_as(C.c_void_p), T, pos, 1, out.ctypes.data_as(C.c_void_p), None))
+        y = np.zeros((T, orow // 4), np.float32)
+        check(lib.ie_b200_engine_read_rows(h, T * row, orow, 0, T, y.ctypes.data_as(C.c_void_p)))
+        return y
+
+    want = chunks(engines[0])  # (also loads the kernels)
+    torch.cuda.synchronize()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - (48 << 20), dtype=torch.uint8, device=cuda)
+    got = chunks(engines[1])
+    del fill
+    torch.cuda.empty_cache()
+    assert np.abs(want).max() > 0.1
+    assert not (got == want).all()  # one split, not several
+    assert np.abs(got - want).max() <= 1.6e-5 * np.abs(want).max()
+    for h in engines:
+        lib.ie_b200_engine_destroy(h)
