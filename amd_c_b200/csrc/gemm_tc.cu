@@ -451,15 +451,24 @@ static uint32_t tc_splits(uint32_t rows, uint32_t nb, uint32_t T) {
   return s < 1u ? 1u : s;
 }
 
-}  // namespace ieb
-
-using namespace ieb;
-
-extern "C" size_t ie_b200_gemm_tc_scratch_bytes(uint32_t rows, uint32_t cols, uint32_t T) {
+// What one call over T tokens takes of the scratch.
+static size_t tc_scratch(uint32_t rows, uint32_t cols, uint32_t T) {
   const uint32_t nb = cols / 32u, nt = (T + TC_TOK - 1) / TC_TOK, splits = tc_splits(rows, nb, T);
   const size_t bp = (size_t)nt * nb * TC_TOK * TC_TOK_STAGE, part = splits > 1u ? (size_t)splits * T * rows * sizeof(float) : 0u;
   const size_t scales = ((size_t)nt * TC_TOK * sizeof(float) + 255u) & ~(size_t)255u;
   return bp + part + scales + 512u;
+}
+
+}  // namespace ieb
+
+using namespace ieb;
+
+// Enough for every call of up to T tokens: fewer token tiles mean more splits along K, so a shorter chunk may take more. (Within a
+// number of token tiles the splits stay the same and the longest takes the most.)
+extern "C" size_t ie_b200_gemm_tc_scratch_bytes(uint32_t rows, uint32_t cols, uint32_t T) {
+  size_t most = tc_scratch(rows, cols, T);
+  for (uint32_t t = TC_TOK; t < T; t += TC_TOK) most = std::max(most, tc_scratch(rows, cols, t));
+  return most;
 }
 
 namespace ieb {
@@ -533,7 +542,7 @@ int ieb::gemm_tc_run(int kind, const void *d_w, uint32_t rows, uint32_t cols, in
   if (rows == 0 || T == 0) return IE_B200_OK;
   if (!aligned16(d_w) || !aligned16(d_xq) || (x_stride & 15u) || (y_stride & 3u) || (res_stride & 3u) || ((uintptr_t)d_scratch & 255u))
     return fail(IE_B200_E_ARG, "ie_b200_gemm_tc: the matrix and the Q8 rows must be 16-byte aligned, strides multiples of 4, the scratch 256-byte aligned");
-  if (scratch_bytes < ie_b200_gemm_tc_scratch_bytes(rows, cols, T)) return fail(IE_B200_E_SIZE, "ie_b200_gemm_tc: scratch of %zu bytes, %zu needed", scratch_bytes, ie_b200_gemm_tc_scratch_bytes(rows, cols, T));
+  if (scratch_bytes < tc_scratch(rows, cols, T)) return fail(IE_B200_E_SIZE, "ie_b200_gemm_tc: scratch of %zu bytes, %zu needed", scratch_bytes, tc_scratch(rows, cols, T));
   const uint32_t nb = cols / 32u, nt = (T + TC_TOK - 1) / TC_TOK, splits = tc_splits(rows, nb, T);
   if (w_exp < -100 || w_exp > 100) return fail(IE_B200_E_ARG, "ie_b200_gemm_tc: weight exponent %d", w_exp);
   uint8_t *bp = static_cast<uint8_t *>(d_scratch);

@@ -53,3 +53,12 @@ def test_attention_chunk_scratch_is_bounded(lib):
         for hd in (64, 128):
             sizes = [size(heads, hd, T) for T in (1, 2, 17, 77, 256, 300, 2048, 8192)]
             assert sizes == sorted(sizes) and sizes[-1] <= 171 << 20
+
+
+def test_gemm_scratch_covers_every_shorter_chunk(lib):
+    """ie_b200_gemm_tc_scratch_bytes(T) is enough for every chunk of up to T tokens (fewer token tiles: more splits along K)."""
+    size = lib.ie_b200_gemm_tc_scratch_bytes
+    for rows, cols in ((5120, 17408), (3072, 8192), (8192, 28672), (4096, 4096), (28672, 4096), (256, 768), (3584, 18944)):
+        ts = [1, 17, 100, 255, 256, 257, 384, 449, 512, 513, 600, 768, 769, 1024, 1536, 2048]
+        sizes = [size(rows, cols, T) for T in ts]
+        assert sizes == sorted(sizes), (rows, cols)

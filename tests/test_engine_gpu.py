@@ -19,7 +19,7 @@ class Engine:
 
         self.lib, self.T, self.arena = _lib.load(), T, arena_bytes
         self.h, self.keep = C.c_void_p(), []
-        d = _lib.EngineDesc(1, 1, 64, 64, 1, T, 16, 1e-5, 0, 0, arena_bytes + 64 * T, arena_bytes, arena_bytes, 64, 8)
+        d = _lib.EngineDesc(1, 1, 64, T, 1, T, 16, 1e-5, 0, 0, arena_bytes + 64 * T, arena_bytes, arena_bytes, 64, 8)
         self.check(self.lib.ie_b200_engine_create(C.byref(d), C.byref(self.h)))
 
     def check(self, r):
@@ -40,14 +40,15 @@ class Engine:
         self.check(self.lib.ie_b200_engine_read_rows(self.h, off, 4 * n, 0, 1, out.ctypes.data_as(C.c_void_p)))
         return out
 
-    def run(self, gemvs):
+    def run(self, gemvs, T=None):
         from amd_c_b200._lib import Op
         from amd_c_b200.backend import OP_GEMV
 
         ops = [Op(OP_GEMV, m, -1, -1, 0, 0, a, b, NONE, NONE, NONE, a_s, b_s, 0, 0, 0) for m, a, a_s, b, b_s in gemvs]
         self.check(self.lib.ie_b200_engine_set_ops(self.h, (Op * len(ops))(*ops), len(ops), len(ops)))
-        toks, out = np.zeros(self.T, np.uint32), np.zeros(self.T, np.uint32)
-        self.check(self.lib.ie_b200_engine_run(self.h, toks.ctypes.data_as(C.c_void_p), self.T, 0, 1, out.ctypes.data_as(C.c_void_p), None))
+        T = T or self.T
+        toks, out = np.zeros(T, np.uint32), np.zeros(T, np.uint32)
+        self.check(self.lib.ie_b200_engine_run(self.h, toks.ctypes.data_as(C.c_void_p), T, 0, 1, out.ctypes.data_as(C.c_void_p), None))
 
     def close(self):
         self.lib.ie_b200_engine_destroy(self.h)
@@ -145,3 +146,24 @@ def test_chunk_without_room_for_the_attention_scratch(cuda):
     assert np.abs(got - want).max() <= 1.6e-5 * np.abs(want).max()
     for h in engines:
         lib.ie_b200_engine_destroy(h)
+
+
+@pytest.mark.parametrize("rows,cols,T_max,T", [(3072, 8192, 384, 256), (3072, 8192, 384, 384)])
+def test_gemm_workspace_holds_for_shorter_chunks(cuda, rows, cols, T_max, T):
+    """The engine's GEMM workspace is sized for its longest chunk; a shorter one may split K more often and take more of it: such
+    chunks run, and equal the multi-token GEMV (1e-5 of the largest output, as test_gemm_tc_matches_gemv)."""
+    import torch
+
+    from amd_c_b200 import kernels as K
+
+    rng = np.random.default_rng(1)
+    xs, ys = 40 * cols // 32, 4 * rows
+    e = Engine(T_max * (xs + ys), T_max)
+    m = K.Mat.from_gguf(synth.GGML_Q4_0, torch.from_numpy(np.ascontiguousarray(synth.q4_0_normal(rng, rows, cols, sigma=0.02))).to(cuda), rows, cols)
+    x = _q8(torch, K, rng, T, cols, cuda)
+    e.write(0, x)
+    e.run([(e.add(m), 0, xs, T_max * xs, ys)], T)
+    got = e.read(T_max * xs, T * rows).reshape(T, rows)
+    want = K.gemv(m, torch.from_numpy(x).to(cuda)).cpu().numpy()
+    assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+    e.close()
