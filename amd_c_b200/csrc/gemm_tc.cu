@@ -22,7 +22,8 @@
 // weights and the tokens' 128 bytes each of activations per 32-column stage, as many stages as fit.
 // Matrices with few rows (3584 x 18944: 14 CTAs) are split along K over grid.z, every split writing its partial sums to
 // scratch, which a second kernel adds in split order (deterministic). Every mbarrier wait is bounded by wall time and reports through the device
-// error word; tensor memory is freed on every path.
+// error word; a warp goes on or gives up as one, and a CTA that gave up waits for its copies and MMAs on their way before it
+// frees its tensor memory and ends.
 //
 // Half precision has a narrow exponent range, so both sides are scaled by exact powers of two before they are split (a value
 // below 2^-14 would lose its low term to the subnormal grid): the weights by 2^S_w, S_w chosen once per matrix from a bound on
@@ -237,15 +238,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
   uint8_t *sB = sA + a.sa * TC_A_STAGE;                    // [stage][4 chunks][hi | lo][tokens][16 B]
   uint8_t *sR = sB + (size_t)a.sb * min(a.T + 15u & ~15u, (uint32_t)TC_TOK) * TC_TOK_STAGE;  // raw weights: two stages per producer warp
   uint64_t *bars = reinterpret_cast<uint64_t *>(sR + TC_PROD_WARPS * 2u * RS_BYTES<KIND>);
-  uint64_t *full_a = bars, *empty_a = bars + TC_MAX_ST, *full_b = bars + 2 * TC_MAX_ST, *empty_b = bars + 3 * TC_MAX_ST, *done = bars + 4 * TC_MAX_ST;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 4 * TC_MAX_ST + 1);
+  uint64_t *full_a = bars, *empty_a = bars + TC_MAX_ST, *full_b = bars + 2 * TC_MAX_ST, *empty_b = bars + 3 * TC_MAX_ST, *done = bars + 4 * TC_MAX_ST,
+           *drained = done + 1;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 4 * TC_MAX_ST + 3);
   __shared__ uint32_t s_abort;
   __shared__ float s_inv[TC_TOK];
 
   if (tid == 0) {
     s_abort = 0u;
     for (int s = 0; s < TC_MAX_ST; s++) mbar_init(&full_a[s], (uint32_t)TC_PROD_WARPS), mbar_init(&empty_a[s], n_tiles), mbar_init(&full_b[s], 1u), mbar_init(&empty_b[s], n_tiles);
-    mbar_init(done, n_tiles);
+    mbar_init(done, n_tiles), mbar_init(&drained[0], 1u), mbar_init(&drained[1], 1u);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == TC_PROD_WARPS) {  // tensor memory: all 512 columns (two accumulators of up to 256 columns), by one warp
@@ -269,6 +271,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
   for (uint32_t j = tid; j < TC_TOK; j += TC_THREADS) s_inv[j] = nt * TC_TOK + j < a.T ? __fmul_rn(a.tok_inv[nt * TC_TOK + j], a.w_inv) : 0.0f;
   __syncthreads();
 
+  bool gave_up = false;   // of a thread that issues MMAs
+  uint32_t issued = 0;    // stages asked for by the thread that copies the activations
   if (warp < TC_PROD_WARPS) {
     // ---------------- producers ----------------
     const uint32_t r = lane & 15u, hf = (uint32_t)lane >> 4, rl = ((uint32_t)warp & 7u) * 16u + r;  // row of the raw stage, column half, row in the tile
@@ -285,7 +289,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
       }
       uint32_t hi[8], lo[8];
       tc_convert<KIND>(src, r, i, b, hf, a.w_scale, hi, lo);
-      if (!mbar_wait(&empty_a[s], par, &s_abort)) break;
+      if (!__all_sync(0xFFFFFFFFu, mbar_wait(&empty_a[s], par, &s_abort))) break;  // the warp goes on or gives up as one
       uint8_t *dst = sA + s * TC_A_STAGE + dst0;
 #pragma unroll
       for (int c = 0; c < 2; c++) {  // 8-column chunks 2 hf + c of the block
@@ -298,9 +302,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
       if (++s == a.sa) s = 0u, par ^= 1u;
     }
     // ---------------- epilogue: accumulators -> token rows ----------------
-    const bool finished = mbar_wait(done, 0u, &s_abort);
+    const bool finished = __all_sync(0xFFFFFFFFu, mbar_wait(done, 0u, &s_abort));
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (finished && !s_abort) {
+    if (finished) {
       // warp w reads lanes 32 (w & 3) .. + 31 of tensor memory (a warp reaches the quarter w mod 4 only): tile (w >> 2) & 1,
       // token columns 32 (w >> 3) + 64 k ..
       const uint32_t q = (uint32_t)warp & 3u, te = ((uint32_t)warp >> 2) & 1u, ch = (uint32_t)warp >> 3;
@@ -354,7 +358,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
       const uint64_t b_j = lbo >> 3, b_lo = n_eff;
       uint32_t s = 0, pa = 0, sb = 0, pb = 0;
       for (uint32_t it = 0; it < n_it; it++) {
-        if (!mbar_wait(&full_a[s], pa, &s_abort) || !mbar_wait(&full_b[sb], pb, &s_abort)) break;
+        if (!mbar_wait(&full_a[s], pa, &s_abort) || !mbar_wait(&full_b[sb], pb, &s_abort)) {
+          gave_up = true;
+          break;
+        }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint64_t da = da0 + s * (uint32_t)(TC_A_STAGE >> 4), db = db0 + sb * (b_stage >> 4);
         const uint32_t acc = it ? 1u : 0u;
@@ -369,12 +376,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
         if (++s == a.sa) s = 0u, pa ^= 1u;
         if (++sb == a.sb) sb = 0u, pb ^= 1u;
       }
-      tc_commit(done);
+      if (!gave_up) tc_commit(done);  // (never both tiles' after giving up: the epilogue reads whole results only)
     }
   } else {
     // ---------------- activations: one bulk copy per stage ----------------
     if (lane == 0) {
-      uint32_t issued = 0;
       for (uint32_t it = 0; it < n_it; it++) {
         const uint32_t s = it % a.sb, round = it / a.sb;
         if (round > 0 && !mbar_wait(&empty_b[s], (round - 1u) & 1u, &s_abort)) break;
@@ -382,21 +388,20 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
         bulk_g2s(sB + s * b_stage, a.bp + (size_t)nt * a.nb * TC_TOK * TC_TOK_STAGE + (size_t)(kb0 + it) * b_stage, b_stage, &full_b[s]);
         issued = it + 1u;
       }
-      if (s_abort) {  // gave up: do not leave while copies are still on their way into this CTA's shared memory
-        for (uint32_t it = issued > a.sb ? issued - a.sb : 0u; it < issued; it++) {
-          const uint64_t t0 = tc_now();
-          uint32_t ok = 0;
-          while (!ok && tc_now() - t0 < 10000000ull)
-            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-                         : "=r"(ok) : "r"(smem_u32(&full_b[it % a.sb])), "r"((it / a.sb) & 1u) : "memory");
-        }
-      }
     }
   }
   if (warp < TC_PROD_WARPS) asm volatile("cp.async.wait_group 0;" ::: "memory");  // (after giving up: none is left on its way)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (tid == 0 && s_abort && a.err) atomicExch(a.err, 5u);
+  if (s_abort) {  // (nobody sets it any more) do not leave while MMAs or copies still use this CTA's memory
+    if (lane == 0 && warp >= TC_PROD_WARPS && warp < TC_PROD_WARPS + 2 && (uint32_t)warp - TC_PROD_WARPS < n_tiles) {
+      uint64_t *bar = &drained[warp - TC_PROD_WARPS];
+      tc_commit(bar), mbar_drain(bar, 0u);
+    }
+    for (uint32_t it = issued > a.sb ? issued - a.sb : 0u; it < issued; it++) mbar_drain(&full_b[it % a.sb], (it / a.sb) & 1u);
+    if (tid == 0 && a.err) atomicExch(a.err, 5u);
+    __syncthreads();
+  }
   __syncwarp();
   if (warp == TC_PROD_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
