@@ -155,6 +155,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
 
   // positions of this split: whole blocks of 128, dealt evenly (read by each role where it first needs them: the Q rows do not)
   uint32_t pos0 = 0u, p_hi = 0u, b0 = 0u, n = 0u;
+  uint32_t issued = 0u;  // blocks asked for by the loader
   auto positions = [&] {
     pos0 = *a.pos, p_hi = pos0 + row_token(min(rows_total, row0 + 128u * a.tiles) - 1u, a.inv_g) + 1u;
     const uint32_t blocks = (p_hi + PT_KEYS - 1u) / PT_KEYS, per = (blocks + gridDim.z - 1u) / gridDim.z;
@@ -479,20 +480,11 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
           }
         }
       }
-      if (!ok) {  // gave up: do not leave while MMAs still read this CTA's shared memory
-        tc_commit(drained);
-        const uint64_t t0 = tc_now();
-        uint32_t done = 0;
-        while (!done && tc_now() - t0 < 10000000ull)
-          asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-                       : "=r"(done) : "r"(smem_u32(drained)), "r"(0u) : "memory");
-      }
     }
   } else {
     // ---------------- loader: K and V blocks into the ring ----------------
     positions();
     const uint32_t total = 2u * n, head_row = g * a.kv_len;
-    uint32_t issued = 0;
     for (uint32_t u = 0; u < total; u++) {
       const uint32_t round = u / PT_RING, buf = u % PT_RING, k0 = (b0 + (u >> 1)) * PT_KEYS, rows = min((uint32_t)PT_KEYS, p_hi - k0);
       if (!__all_sync(0xFFFFFFFFu, round == 0u || mbar_wait(&kv_empty[buf], (round - 1u) & 1u, &s_abort))) break;
@@ -519,20 +511,33 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
         if (lane == 0) mbar_arrive(&kv_full[buf]);
       }
     }
-    if (s_abort && lane == 0) {  // gave up: do not leave while copies are on their way into this CTA's shared memory
-      const uint64_t t0 = tc_now();
-      for (uint32_t u = issued > PT_RING ? issued - PT_RING : 0u; u < issued; u++) {
-        const bool ragged = (u & 1u) && p_hi - (b0 + (u >> 1)) * PT_KEYS < PT_KEYS;
-        uint32_t done = 0;
-        while (!done && tc_now() - t0 < 10000000ull)
-          asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
-                       : "=r"(done) : "r"(smem_u32(ragged ? tail : &kv_full[u % PT_RING])), "r"(ragged ? 0u : (u / PT_RING) & 1u) : "memory");
-      }
-    }
   }
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && s_abort && a.err) atomicExch(a.err, 5u);
+  if (s_abort) {  // (nobody sets it any more) do not leave while MMAs or copies still use this CTA's memory
+    if (warp == PT_SOFT_WARPS && lane == 0) tc_commit(drained), mbar_drain(drained, 0u);
+    if (warp == PT_SOFT_WARPS + 1 && lane == 0) {
+      for (uint32_t u = issued > PT_RING ? issued - PT_RING : 0u; u < issued; u++) {
+        const bool ragged = (u & 1u) && p_hi - (b0 + (u >> 1)) * PT_KEYS < PT_KEYS;
+        mbar_drain(ragged ? tail : &kv_full[u % PT_RING], ragged ? 0u : (u / PT_RING) & 1u);
+      }
+    }
+    // The rows say so too (a caller may have given no error word): NaN, in the outputs or in the records that the merge reads.
+    const float nan = __int_as_float(0x7FFFFFFF);
+    const uint32_t n_rows = min(rows_total - row0, 128u * a.tiles), nbq = a.n_head * HD / 32u;
+    for (uint32_t i = threadIdx.x; i < n_rows * (HD / 32u); i += PT_THREADS) {
+      const uint32_t r = row0 + i / (HD / 32u), tok = row_token(r, a.inv_g), head = g * a.G + (r - tok * a.G), b = i % (HD / 32u);
+      if (a.part) {
+        if (b < 2u) a.ml[(split * (size_t)a.T * a.n_head + (size_t)tok * a.n_head + head) * 2u + b] = nan;
+      } else {
+        float *row = reinterpret_cast<float *>(reinterpret_cast<char *>(a.out) + a.out_stride * tok) + (size_t)head * HD + 32u * b;
+        for (int e = 0; e < 32; e++) row[e] = nan;
+        if (a.oq) reinterpret_cast<float *>(a.oq + a.oq_stride * tok + 32u * (size_t)nbq)[head * (HD / 32u) + b] = nan;
+      }
+    }
+    if (threadIdx.x == 0 && a.err) atomicExch(a.err, 5u);
+    __syncthreads();
+  }
   __syncwarp();
   if (warp == PT_SOFT_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
