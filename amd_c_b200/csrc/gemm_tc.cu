@@ -263,8 +263,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
   // its way before the wait for the activations
   const uint32_t t_p = (uint32_t)warp >> 3, row0 = m0 + t_p * 128u + ((uint32_t)warp & 7u) * 16u;
   uint8_t *raw = sR + (uint32_t)warp * 2u * RS_BYTES<KIND>;
+  const uint32_t kq = kb0 & ~3u;  // raw stages start at multiples of four blocks; a split may start inside one
   if (warp < TC_PROD_WARPS) {
-    if (n_it > 0u) rs_issue<KIND>(a.w, a.rowb, a.rows, a.nb, rs_smem(raw), row0, kb0, lane);
+    if (n_it > 0u) rs_issue<KIND>(a.w, a.rowb, a.rows, a.nb, rs_smem(raw), row0, kq, lane);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   pdl_wait();  // the expanded activations (and the residual) are complete
@@ -279,12 +280,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
     const uint32_t dst0 = t_p * 2 * TC_A_TILE + (rl >> 3) * 128u + (rl & 7u) * 16u + hf * 2u * 2048u;
     uint32_t s = 0, par = 1u;  // the first round finds every stage empty
     for (uint32_t it = 0; it < n_it; it++) {
-      const uint32_t i = it & 3u, b = kb0 + it;
-      const uint8_t *src = raw + ((it >> 2) & 1u) * RS_BYTES<KIND>;
-      if (i == 0u) {  // the next four blocks have arrived; ask for the four after them, whose place all lanes have done with
+      const uint32_t b = kb0 + it, i = b & 3u, q = (b - kq) >> 2;  // block, its place in raw stage q
+      const uint8_t *src = raw + (q & 1u) * RS_BYTES<KIND>;
+      if (i == 0u || it == 0u) {  // the next four blocks have arrived; ask for the four after them, whose place all lanes have done with
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncwarp();
-        if (it + 4u < n_it) rs_issue<KIND>(a.w, a.rowb, a.rows, a.nb, rs_smem(raw + (((it >> 2) + 1u) & 1u) * RS_BYTES<KIND>), row0, b + 4u, lane);
+        if (kq + 4u * q + 4u < kb1) rs_issue<KIND>(a.w, a.rowb, a.rows, a.nb, rs_smem(raw + ((q + 1u) & 1u) * RS_BYTES<KIND>), row0, kq + 4u * q + 4u, lane);
         asm volatile("cp.async.commit_group;" ::: "memory");
       }
       uint32_t hi[8], lo[8];
@@ -561,8 +562,9 @@ int ieb::gemm_tc_run(int kind, const void *d_w, uint32_t rows, uint32_t cols, in
   }
   TcArgs a = {};
   a.w = static_cast<const uint8_t *>(d_w), a.rowb = row_bytes_of(kind, cols), a.rows = rows, a.nb = nb, a.T = T;
+  // (not rounded up to whole raw stages: a longer accumulation loses more, 4096 x 4096 Q4_0 above 128 tokens 1.60e-6 against 64 bits with
+  // 15 blocks per split, 1.74e-6 with 16)
   a.blocks_per_split = (nb + splits - 1u) / splits;
-  a.blocks_per_split = (a.blocks_per_split + 3u) & ~3u;  // whole raw stages
   a.bp = bp, a.y = d_y, a.bias = d_bias, a.res = d_res, a.ys = y_stride, a.rs = res_stride, a.partial = partial, a.err = d_err;
   a.w_scale = ldexpf(1.0f, w_exp), a.w_inv = ldexpf(1.0f, -w_exp), a.tok_inv = tok_inv;
   const uint32_t used_splits = (nb + a.blocks_per_split - 1u) / a.blocks_per_split;

@@ -642,7 +642,10 @@ def test_gemm_matches_gemv(ora, cuda, typ, rows, cols, T):
                                              (synth.GGML_Q4_0, 130, 320, 20), (synth.GGML_Q4_0, 5000, 4096, 300), (synth.GGML_Q6_K, 300, 18944, 64),
                                              (synth.GGML_Q4_K, 9000, 3584, 256), (synth.GGML_Q4_0, 1, 64, 1), (synth.GGML_Q8_0, 1000, 4096, 100),
                                              (synth.GGML_Q8_0, 77, 192, 33), (synth.GGML_Q8_0, 4096, 14336, 256), (synth.GGML_Q4_0, 1001, 4096, 40),
-                                             (synth.GGML_Q6_K, 130, 2048, 129), (synth.GGML_Q8_0, 300, 32 * 38, 128)])
+                                             (synth.GGML_Q6_K, 130, 2048, 129), (synth.GGML_Q8_0, 300, 32 * 38, 128),
+                                             # splits along K that start inside a raw stage of four blocks (15, 9 and 15, 43 blocks each)
+                                             (synth.GGML_Q4_0, 4096, 4096, 130), (synth.GGML_Q8_0, 257, 32 * 142, 40), (synth.GGML_Q6_K, 4000, 4096, 200),
+                                             (synth.GGML_Q4_K, 12000, 4096, 17)])
 def test_gemm_tc_matches_gemv(ora, cuda, typ, rows, cols, T):
     """The prompt-chunk GEMM on tcgen05 / tensor memory (both operands as two half-precision terms, fp32 accumulation over the
     whole K in tensor memory) against the multi-token GEMV, which is bit-exact with the CPU reference: 1e-5 of the largest
