@@ -149,7 +149,8 @@ __global__ void __launch_bounds__(256) tc_expand_kernel(const uint8_t *xq, size_
 // ---- weights: half a block (16 columns) of one row of a raw stage -> two f16 terms, column pairs (0, 2), (1, 3) per word ----
 // Q4_0, Q8_0, Q6_K: the integer weight is exact in f16 (a byte ORed into 0x6400 is 1024 + byte), and so is the rest of a
 // product of two halves, which one fma gives: hi = rn(s q), lo = s q - hi, two weights per instruction. A Q6_K scale d sc has
-// 19 bits: s = s_hi + s_lo, lo = (s_hi q - hi) + s_lo q. Q4_K (d sc q - dmin mn cancels) is worked in f32 and split after.
+// 19 bits: s = s_hi + s_lo, lo = (s_hi q - hi) + s_lo q, the last product as (2^10 s_lo) (2^-10 q): of a super-block far below the
+// matrix's largest, s_lo alone would lie on the subnormal grid. Q4_K (d sc q - dmin mn cancels) is worked in f32 and split after.
 // About 2 (Q4_0) to 5 (Q4_K) instructions per weight; converting each to f32, scaling and splitting there took more than 10.
 __device__ __forceinline__ uint32_t h2u(__half2 h) { return *reinterpret_cast<const uint32_t *>(&h); }
 __device__ __forceinline__ __half2 u2h(uint32_t u) { return *reinterpret_cast<const __half2 *>(&u); }
@@ -191,14 +192,15 @@ __device__ __forceinline__ void tc_convert(const uint8_t *raw, uint32_t r, uint3
     const float df = h2f(*reinterpret_cast<const uint16_t *>(raw + 1664u + 4u * r + 2u * ((b >> 3) & 1u)));
     const float s = __fmul_rn(__fmul_rn(df, (float)(int8_t)sc), w_scale);
     const __half sh = __float2half_rn(s);
-    const __half2 s_hi = __half2half2(sh), s_lo = __float2half2_rn(s - __half2float(sh)), off = u2h(0x64206420u);  // 1056
+    const __half2 s_hi = __half2half2(sh), s_lo = __float2half2_rn(1024.0f * (s - __half2float(sh))), off = u2h(0x64206420u);  // 1056
+    const __half2 down = u2h(0x14001400u), off_d = u2h(0xBC20BC20u);  // 2^-10, -1056 2^-10
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       const uint32_t w6 = (v[k] & 0x0F0F0F0Fu) | (((hw >> (2 * k)) & 0x03030303u) << 4);
 #pragma unroll
       for (int p = 0; p < 2; p++) {
-        const __half2 q = __hsub2(u2h(((w6 >> (8 * p)) & 0x003F003Fu) | 0x64006400u), off), h = __hmul2(s_hi, q);
-        hi[2 * k + p] = h2u(h), lo[2 * k + p] = h2u(__hfma2(s_lo, q, __hfma2(s_hi, q, __hneg2(h))));
+        const __half2 x = u2h(((w6 >> (8 * p)) & 0x003F003Fu) | 0x64006400u), q = __hsub2(x, off), h = __hmul2(s_hi, q);
+        hi[2 * k + p] = h2u(h), lo[2 * k + p] = h2u(__hfma2(s_lo, __hfma2(x, down, off_d), __hfma2(s_hi, q, __hneg2(h))));
       }
     }
   } else {

@@ -698,6 +698,26 @@ def test_gemm_tc_small_and_large_weights(ora, cuda):
         assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max(), sigma
 
 
+def test_gemm_tc_q6_k_blocks_of_very_different_scale(ora, cuda):
+    """Q6_K super-blocks 2^18 below the matrix's largest (whose activations are zero): the result equals the GEMV's to 1e-5 as elsewhere.
+    (Weights are split into halves on a grid of 2^-24 where the matrix's largest is 8192: an error of half a unit is 2e-6 of the
+    root mean square of these weights. An error of 16 units, a scale on that grid times a weight of 32, is 4e-5 of it.)"""
+    from amd_c_b200 import kernels as K
+
+    rng = np.random.default_rng(17)
+    rows, cols, T = 200, 1024, 40
+    raw = synth.make_gguf_bytes(synth.GGML_Q6_K, rng, rows, cols).reshape(rows, cols // 256, 210).copy()
+    d = (2.0 ** -8 * (1.0 + rng.random((rows, cols // 256)))).astype(np.float16)
+    d[:, 0] = 1024.0
+    raw[:, :, 208:210] = d[..., None].view(np.uint8)
+    m = K.Mat.from_gguf(synth.GGML_Q6_K, dev(raw.reshape(-1), cuda), rows, cols)
+    x = rng.standard_normal((T, cols)).astype(np.float32)
+    x[:, :256] = 0.0
+    xq = K.quant_q8(dev(x, cuda))
+    want, got = K.gemv(m, xq).cpu().numpy(), K.gemm_tc(m, xq).cpu().numpy()
+    assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+
+
 @pytest.mark.parametrize("n_head,n_kv,hd,T,pos0", [(8, 2, 128, 9, 70), (28, 4, 128, 5, 200), (8, 8, 64, 19, 0), (10, 2, 64, 4, 129), (16, 2, 128, 3, 63),
                                                           (24, 8, 128, 11, 100), (12, 2, 64, 7, 300)])
 def test_attention_prefill_chunk(ora, cuda, n_head, n_kv, hd, T, pos0):
