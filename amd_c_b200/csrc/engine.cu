@@ -129,6 +129,7 @@ int ar_norm_reduce(ie_b200_allreduce *a, const float *d_part, const float *d_res
                    uint32_t n, uint32_t *d_err, cudaStream_t st, bool pushed);
 void ar_push_info(const ie_b200_allreduce *a, ArPush *out);  // allreduce.cu
 bool ar_connected(const ie_b200_allreduce *a);
+uint32_t gemv_tokens_phases(int kind, uint32_t cols);  // gemv_tokens.cu
 int gemm_tc_run(int kind, const void *d_w, uint32_t rows, uint32_t cols, int w_exp, const void *d_xq, float *d_y, const float *d_bias, const float *d_res, uint32_t T,
                 size_t x_stride, size_t y_stride, size_t res_stride, void *d_scratch, size_t scratch_bytes, uint32_t *d_err, cudaStream_t st, bool act_ready);  // gemm_tc.cu
 int attn_decode_fused(const float *d_q, const float *d_k, const float *d_v, void *d_kc, void *d_vc, const float *d_cos, const float *d_sin, float *d_out,
@@ -140,11 +141,16 @@ int attn_decode_fused(const float *d_q, const float *d_k, const float *d_v, void
 static bool stream_ok(const EMat &m) { return gemv_direct_ok(m.kind, m.cols); }
 
 // A few tokens above sixteen: two passes of the multi-token GEMV over the weights, or one of the tcgen05 GEMM, whose products cost
-// about the same from 17 to 100 tokens? Up to 24 tokens (the second pass has one token tile) the GEMV is ahead where its
-// activations stay in shared memory: 28672 x 4096 Q4_0 56 .. 58 against 71 us, 6144 x 4096 20 .. 21 / 23, 2048 x 2048 Q8_0 8 / 13,
-// 37888 x 3584 Q4_K 70 .. 72 / 76; not for long rows (4096 x 14336 42 .. 47 / 39 .. 40, 2048 x 8192 Q8_0 21 .. 23 / 19 .. 20) nor for
-// Q6_K, two tensor products per block (2048 x 4096 15 .. 16 / 15); at 28 tokens it is level (66 / 71, 20 / 19, 83 / 77).
-static bool few_tokens(const EMat &m, uint32_t T) { return T <= 24u && m.cols <= 6144u && m.kind != IE_B200_MAT_Q6K; }
+// about the same from 17 to 100 tokens? Up to 24 tokens (the second pass has one token tile) the GEMV is ahead where the activations
+// of a row stay in shared memory: 28672 x 4096 Q4_0 56 .. 58 against 69 us, x 5120 64 .. 66 / 86, Q4_K 62 .. 63 / 82 and 74 .. 76 /
+// 102, Q8_0 x 2048 36 .. 37 / 39. Where they do not, every 16-row tile stages them anew: ahead only while a half CTA has one
+// tile, and not for long rows (Q8_0 4096 x 4096 14 .. 15 / 17 .. 18, x 5120 18 .. 19 / 20, but 6144 x 4096 23 .. 24 / 22 .. 23, 28672 x
+// 4096 84 / 74; 2048 x 6144 16 .. 18 / 15 .. 16). Not for Q6_K, two tensor products per block (2048 x 4096 15 .. 16 / 15); at 28
+// tokens it is level.
+static bool few_tokens(const EMat &m, uint32_t T) {
+  if (T > 24u || m.kind == IE_B200_MAT_Q6K || m.kind == IE_B200_MAT_F32) return false;
+  return gemv_tokens_phases(m.kind, m.cols) == 1u || (m.rows <= 32u * (uint32_t)sm_count() && m.cols <= 5120u);
+}
 
 // Does the tcgen05 GEMM run op o over T tokens? (From the reference's threshold on, src/hip.c:965.) The one place that says so:
 // launch_op dispatches by it, and tc_same_act relies on it to know what the scratch holds.

@@ -15,7 +15,7 @@
 //
 // Memory: each warp streams its own blocks through a private ring of cp.async stages (16 rows x 4 blocks each, no barrier
 // among warps; ldmatrix hands thread (g, t) word t of row g, which is the A fragment's word), so that 16 warps x 5 stages =
-// 90 KB per SM are in flight; the first stages are asked for before the kernel waits for its predecessor. The activations of a
+// 90 KB per SM are in flight (Q4_0, up to 8 tokens; 3 stages behind the one being worked for Q6_K, Q8_0 and above 8 tokens); the first stages are asked for before the kernel waits for its predecessor. The activations of a
 // CTA are staged in the order of the B fragments; rows longer than fit are worked in phases over the columns.
 #include <algorithm>
 
@@ -289,12 +289,34 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemv_tokens_kernel(const GtArgs
   }
 }
 
+// Shared memory of the rings and the reduction, of a block's activations, and blocks whose activations fit beside the former.
+template <int KIND, int NT>
+struct GtFit {
+  static constexpr uint32_t fixed = 2u * (8u * GT_STAGES<KIND, NT> * RS_BYTES<KIND> + GT_RED), per = NT * (256u + GtKind<KIND>::DS);
+  static constexpr uint32_t cap = (GT_SMEM - fixed) / per / 32u * 32u;
+  static_assert(cap >= 32u, "a phase is at least 32 blocks");
+};
+template <int KIND, int NT>
+static uint32_t gt_phases(uint32_t nb) {
+  return (((nb + 31u) & ~31u) + GtFit<KIND, NT>::cap - 1u) / GtFit<KIND, NT>::cap;
+}
+// Phases over the columns of a pass of sixteen tokens (5120 columns fit for Q4_0 and Q4_K, 3072 for Q6_K, 2048 for Q8_0): with more
+// than one, every 16-row tile stages its activations anew.
+uint32_t gemv_tokens_phases(int kind, uint32_t cols) {
+  const uint32_t nb = cols / 32u;
+  switch (kind) {
+    case IE_B200_MAT_Q4: return gt_phases<IE_B200_MAT_Q4, 2>(nb);
+    case IE_B200_MAT_Q8: return gt_phases<IE_B200_MAT_Q8, 2>(nb);
+    case IE_B200_MAT_Q4K: return gt_phases<IE_B200_MAT_Q4K, 2>(nb);
+    default: return gt_phases<IE_B200_MAT_Q6K, 2>(nb);
+  }
+}
+
 template <int KIND, int NT>
 static int launch_tokens(GtArgs a, cudaStream_t st) {
-  constexpr uint32_t fixed = 2u * (8u * GT_STAGES<KIND, NT> * RS_BYTES<KIND> + GT_RED), per = NT * (256u + GtKind<KIND>::DS);
+  constexpr uint32_t fixed = GtFit<KIND, NT>::fixed, per = GtFit<KIND, NT>::per;
   // the fewest phases whose activations fit beside the rings, all of about the same length
-  const uint32_t cap = (GT_SMEM - fixed) / per / 32u * 32u, up = (a.nb + 31u) & ~31u, phases = (up + cap - 1u) / cap;
-  static_assert((GT_SMEM - fixed) / per >= 32u, "a phase is at least 32 blocks");
+  const uint32_t up = (a.nb + 31u) & ~31u, phases = gt_phases<KIND, NT>(a.nb);
   a.P = (up / 32u + phases - 1u) / phases * 32u;
   const size_t smem = fixed + (size_t)a.P * per;
   auto k = gemv_tokens_kernel<KIND, NT>;

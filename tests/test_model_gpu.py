@@ -194,6 +194,31 @@ def test_prompt_chunks_on_the_half_cache(cuda, ora, name):
         assert nxt == first
 
 
+@pytest.mark.parametrize("T", [17, 20, 24, 25])
+@pytest.mark.parametrize("name", ["tiny-128", "tiny-k", "tiny-q8"])
+def test_chunks_around_the_gemv_gemm_line(cuda, ora, name, T):
+    """Chunks of 17 to 25 tokens: where the multi-token GEMV hands over to the tcgen05 GEMM, and where one layer may use both (Q4_K and
+    Q6_K matrices over the same activations). Every token's logits against the oracle with the same half rounding at the cache store
+    (2e-2 of the logit scale, as the chunks of 32 above), and the choices where the oracle's top-two gap allows."""
+    from oracle.oracle import OracleModel
+
+    cfg = gguf.make_model(gguf.config(name), seed=0)
+    toks = [int(t) for t in np.random.default_rng(T).integers(0, cfg.vocab, T)]
+    om = OracleModel(ora, cfg, 64, kv_f16=True)
+    want = [om.step(t, pos)[1].copy() for pos, t in enumerate(toks)]
+    om.close()
+    b = Backend(cfg, 64, T=32)
+    out = b.run(0, toks, 0, last_only=False)
+    rows = b.read_rows("logits", 0, T).view(np.float32)[:, : cfg.vocab]
+    b.close()
+    for t in range(T):
+        d = float(np.abs(rows[t] - want[t]).max())
+        assert d <= 2e-2 * float(np.abs(want[t]).max()), (t, d)
+        top2 = np.sort(want[t])[-2:]
+        if top2[1] - top2[0] > 2 * d:
+            assert int(out[t]) == int(np.argmax(want[t])), t
+
+
 VARIANTS = [{"IE_B200_PDL": "0"}, {"IE_B200_ATTN_FUSE": "0"}, {"IE_B200_NORM": "tail"}, {"IE_B200_NORM": "prologue"}, {"IE_B200_ATTN": "scalar"}, {"IE_B200_ATTN": "single"},
             {"IE_B200_GEMM": "0"}, {"IE_B200_GEMM": "mma"}, {"IE_B200_PREFILL_ATTN": "0"}, {"IE_B200_STEP": "auto"}, {"IE_B200_SWIGLU": "gemv"}]
 
