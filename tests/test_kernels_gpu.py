@@ -71,8 +71,8 @@ def test_quant_q8_bit_exact(ora, cuda, golden_kernels):
 
 
 def test_quant_q8_rounding_boundaries(ora, cuda):
-    """Values within a few ulps of every k + 0.5 boundary, for several scales: the kernel's reciprocal fast path
-    must fall back to the exact division there and agree with the CPU quantiser bit for bit."""
+    """Values within a few ulps of every k + 0.5 boundary, for several scales: the kernel's quotients, a multiplication by the
+    reciprocal and two fused multiply-adds, are correctly rounded and agree with the CPU quantiser's division bit for bit."""
     from amd_c_b200 import kernels as K
 
     rng = np.random.default_rng(9)
@@ -91,6 +91,25 @@ def test_quant_q8_rounding_boundaries(ora, cuda):
     got = K.quant_q8(dev(x, cuda)).cpu().numpy()
     for t in range(x.shape[0]):
         assert (got[t] == ora.quant_q8(x[t])).all(), t
+
+
+def test_quant_q8_tiny_scales(ora, cuda):
+    """Blocks whose scale lies around the bound below which quotients are worked scaled by 2^100 (1e-25), and down through the
+    denormals to the smallest: the CPU quantiser's bits. (A scale that rounds to nothing gives zeros.)"""
+    from amd_c_b200 import kernels as K
+
+    rng = np.random.default_rng(23)
+    rows = []
+    for top in (1.3e-22, 127e-25, 1.2699e-23, 1.2701e-23, 1e-25, 3e-30, 1.5e-36, 1.1754944e-38, 2e-39, 3e-41, 2.66e-43, 1.9e-43, 1.3e-43, 8.9e-44, 1e-44, 1.4e-45):
+        x = (rng.uniform(-1, 1, 256) * top).astype(np.float32)
+        x[::32] = np.float32(top) * rng.choice([-1, 1], 8)
+        k = (np.arange(7) + 0.5) * np.float32(top) / 127  # half-way values of the block's own scale
+        x[1:8] = k
+        rows.append(x)
+    x = np.stack(rows)
+    got = K.quant_q8(dev(x, cuda)).cpu().numpy()
+    for t in range(x.shape[0]):
+        assert (got[t] == ora.quant_q8(x[t])).all(), float(np.abs(x[t]).max())
 
 
 def test_quant_q8_empty(cuda, lib):
@@ -878,8 +897,8 @@ def test_gemv_several_tokens_one_pass(ora, cuda, typ, rows, cols, T):
     (synth.GGML_Q8_0, 16, 32 * 450, 13), (synth.GGML_Q4_0, 4801, 256, 6), (synth.GGML_Q4_K, 4752, 256, 4), (synth.GGML_Q6_K, 4737, 256, 10),
     (synth.GGML_Q4_K, 31, 18944, 8), (synth.GGML_Q6_K, 18, 18944, 16), (synth.GGML_Q4_0, 20, 1024, 19)])
 def test_gemv_tokens_edges(ora, cuda, typ, rows, cols, T):
-    """The multi-token GEMV where it can go wrong: rows off the 16-row tiles, more tiles than the grid has slots, rows of one
-    block, of blocks that are no multiple of a stage's four, of several activation phases, both token tiles ragged."""
+    """The multi-token GEMV where it can go wrong: rows off the 16-row tiles, more tiles than the grid has slots, rows of two
+    blocks, of blocks that are no multiple of a stage's four, of several activation phases, both token tiles ragged."""
     from amd_c_b200 import kernels as K
 
     rng = np.random.default_rng(rows * 5 + T)
@@ -893,6 +912,29 @@ def test_gemv_tokens_edges(ora, cuda, typ, rows, cols, T):
     y = K.gemv(m, dev(xq, cuda), bias=dev(bias, cuda)).cpu().numpy()
     for t in range(T):
         assert (bits(y[t]) == bits(ora.gemv(kind, qw, qs, rows, cols, xq[t], bias=bias))).all(), t
+
+
+@pytest.mark.parametrize("typ", [synth.GGML_Q4_0, synth.GGML_Q8_0])
+@pytest.mark.parametrize("rows,nb,T", [(5, 1, 2), (17, 3, 9), (33, 33, 16), (40, 511, 6)])
+def test_gemv_tokens_odd_blocks(ora, cuda, typ, rows, nb, T):
+    """The multi-token GEMV over rows of an odd number of blocks, one among them: the Q8 rows of the tokens, 40 bytes a block, lie at
+    the next multiple of 16 (the stride the entry asks for); every token's row bit for bit the CPU's."""
+    import torch
+
+    from amd_c_b200 import kernels as K
+
+    cols = 32 * nb
+    rng = np.random.default_rng(nb * 7 + T)
+    raw = synth.make_gguf_bytes(typ, rng, rows, cols)
+    kind, qw, qs = ora.repack(typ, raw, rows, cols)
+    m = K.Mat.from_gguf(typ, dev(raw, cuda), rows, cols)
+    x = rng.standard_normal((T, cols)).astype(np.float32)
+    xq = np.stack([ora.quant_q8(x[t]) for t in range(T)])
+    buf = torch.zeros((T, (40 * nb + 15) // 16 * 16), dtype=torch.uint8, device=cuda)
+    buf[:, : 40 * nb] = dev(xq, cuda)
+    y = K.gemv(m, buf).cpu().numpy()
+    for t in range(T):
+        assert (bits(y[t]) == bits(ora.gemv(kind, qw, qs, rows, cols, xq[t]))).all(), t
 
 
 def test_allreduce_missing_rank_gives_up(cuda, lib):

@@ -27,9 +27,9 @@ def main():
     cfg = gguf.make_model(gguf.config(model), seed=0)
     kv_f32 = mode == "graph"  # the persistent kernel runs on the half cache
     n_ctx, n_gen, prompt = 160, 40, [1, 2, 3]
-    tpb = TensorParallelBackend(Backend(cfg, n_ctx, T=24, kv_f32=kv_f32, tp=world, rank=rank, device=dev, step_mode=mode), dist.group.WORLD)
+    tpb = TensorParallelBackend(Backend(cfg, n_ctx, T=26, kv_f32=kv_f32, tp=world, rank=rank, device=dev, step_mode=mode), dist.group.WORLD)
     assert tpb.b.step_is_kernel == (mode == "kernel")
-    single = Backend(cfg, n_ctx, T=24, kv_f32=kv_f32, device=dev, step_mode=mode) if rank == 0 else None
+    single = Backend(cfg, n_ctx, T=26, kv_f32=kv_f32, device=dev, step_mode=mode) if rank == 0 else None
     mine = np.zeros(cfg.vocab // world, np.float32)
     want = np.zeros(cfg.vocab, np.float32)
     tok, n_checked, worst = prompt[0], 0, 0.0
@@ -71,7 +71,8 @@ def main():
             tok, _ = single.step(tok, len(prompt) + 12 + i)
             w.append(tok)
         common = next((i for i, (a, b) in enumerate(zip(out, w)) if int(a) != int(b)), n_gen)
-    # a prompt chunk (T tokens per call, each stop one exchange over T x dim floats) against the unsharded engine's chunk
+    # a prompt chunk (T tokens per call, above the 24 that the multi-token GEMV may take: the tcgen05 GEMM; each stop one exchange
+    # over T x dim floats) against the unsharded engine's chunk
     T = tpb.b.T
     pos0 = len(prompt) + 12  # over the same history on both sides: the teacher-forced steps above (the chained tokens may have parted)
     chunk = (np.arange(T, dtype=np.uint32) * 7 + 3) % cfg.vocab
