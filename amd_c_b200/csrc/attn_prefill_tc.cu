@@ -21,6 +21,17 @@
 // some row of the CTA does not see whole are looked through for infinities and NaN (a value that overflowed the half cache must
 // not reach the tokens before it): they are replaced by zeros, and added at the end to the rows that do see them.
 // O is rescaled lazily: only when a row's maximum has grown by more than 2^8 (p stays far inside f16).
+//
+// Error. The tensor cores cut off what an accumulation loses (2^-25.7 of the accumulator per MMA, measured), so what counts is how
+// many MMAs one accumulation takes. Low terms go first, into an accumulator that is still small: they cost next to nothing for S
+// and at the start of O. An accumulation of O ends after a quarter of a row's blocks (pt_segment) and joins the row's sums, kept in
+// fp32 by the softmax threads: in shared memory, or, for two tiles of heads of 128, which leave no room there, in the row's own
+// memory. With four splits and more nothing joins (the merge adds the splits). Relative error against 64 bits (2-norm, random
+// normal q, k, v, 32 x 8 heads of 128, 256 tokens, at 0 / 256 / 1000 / 8000 / 32000 positions, one split): 2.6e-7 / 4.0e-7 / 9.5e-7 /
+// 4.9e-6 / 1.9e-5; high and low terms in turn and one accumulation: 5.2e-7 / 1.3e-6 / 3.0e-6 / 2.0e-5 / 7.5e-5; the mma.sync form
+// (attn_decode.cu's scheme): 4.5e-7 / 7.3e-7 / 1.1e-6 / 5.2e-6 / 1.9e-5. With the splits that the launcher picks: 2.6e-7 / 4.0e-7 /
+// 8.9e-7 / 4.9e-6 / 8.4e-6; 16 tokens at 4000 and 32000 positions 6.8e-7 and 4.8e-6. Exponentials by ex2.approx (2 units in the
+// last place) in place of expf do not show in these figures.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <math.h>
@@ -32,7 +43,7 @@
 
 namespace ieb {
 
-constexpr int PT_SOFT_WARPS = 16, PT_THREADS = (PT_SOFT_WARPS + 2) * 32, PT_RING = 3, PT_KEYS = 128;
+constexpr int PT_RING = 3, PT_KEYS = 128;
 
 struct PtArgs {
   const float *q;
@@ -45,8 +56,7 @@ struct PtArgs {
   float *part;       // [split][T x n_head rows][hd] unnormalised outputs, NULL: one split, final rows written here
   float *ml;         // [split][T x n_head][2] (max in log2 units, sum)
   uint32_t *err;
-  uint32_t wide;     // bit 0: the rows written are 16-byte aligned, bit 1: the q rows are
-  uint32_t tiles;    // 128-row tiles per CTA: 1 or 2
+  uint32_t wide;     // bit 0: the rows written are 16-byte aligned, bit 1: the q rows are, bit 2: the rows written (or the records) are 32-byte aligned
   float inv_g;       // 1 / G
   const __half *vc;  // the V cache (read here only for rows that hold an infinity or a NaN)
 };
@@ -73,6 +83,26 @@ __device__ __forceinline__ uint64_t f32x2_add(uint64_t a, uint64_t b) {
   uint64_t r;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
+}
+
+// Eight neighbouring floats of a row: one 32-byte access (whole sectors, however far apart the lanes' rows lie) where aligned.
+__device__ __forceinline__ void ld8(const float *p, float (&x)[8], bool wide) {
+  if (wide) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]), "=f"(x[6]), "=f"(x[7]) : "l"(p) : "memory");
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; e++) x[e] = p[e];
+  }
+}
+__device__ __forceinline__ void st8(float *p, const uint32_t *v, bool wide) {
+  if (wide) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; e++) p[e] = __uint_as_float(v[e]);
+  }
 }
 
 // Four neighbouring outputs of a (token, head) row per lane, eight lanes per block of 32: the row's floats and its Q8 copy.
@@ -118,12 +148,26 @@ __device__ __forceinline__ uint32_t row_token(uint32_t r, float inv_g) { return 
 template <int HD>
 struct PtSmem {
   static constexpr uint32_t QTERM = 128u * HD * 2u, BLOCK = PT_KEYS * HD * 2u;
-  static constexpr uint32_t Q_OFF = 0u, KV_OFF = 4u * QTERM, BAR_OFF = KV_OFF + PT_RING * BLOCK, PAIR_OFF = BAR_OFF + 256u, TOTAL = PAIR_OFF + 2048u;
+  static constexpr uint32_t Q_OFF = 0u, KV_OFF = 4u * QTERM, BAR_OFF = KV_OFF + PT_RING * BLOCK, PAIR_OFF = BAR_OFF + 256u,
+                            // rows' sums of the segments before: behind everything (heads of 64), in the second tile's Q (heads of 128, one tile)
+                            SUM_OFF = HD == 64 ? PAIR_OFF + 2048u : Q_OFF + 2u * QTERM, TOTAL = PAIR_OFF + 2048u + (HD == 64 ? 2u * 128u * HD * 4u : 0u);
 };
 
+// Blocks of positions that one accumulation in tensor memory takes, of the n that a row tile has in all splits together; f: blocks
+// that every row sees whole. A quarter of them; two (heads of 128: three) blocks that are mostly a diagonal stay together, most of
+// their products are zeros (77 tokens x 32 heads of 128 at 200 positions: 5.3e-7, the mma.sync form 6.9e-7).
 template <int HD>
-__global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const PtArgs a, const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map) {
+__host__ __device__ constexpr uint32_t pt_segment(uint32_t n, uint32_t f) {
+  return n <= (HD == 64 ? 2u : 3u) && f + 1u < n ? n : (n + 3u) / 4u;
+}
+
+// TILES: 128-row tiles of a CTA, eight softmax warps each.
+template <int HD, int TILES>
+__global__ void __launch_bounds__((8 * TILES + 2) * 32, 1) attn_prefill_tc_kernel(const PtArgs a, const __grid_constant__ CUtensorMap k_map,
+                                                                                  const __grid_constant__ CUtensorMap v_map) {
   using L = PtSmem<HD>;
+  constexpr int SOFT_WARPS = 8 * TILES, THREADS = (SOFT_WARPS + 2) * 32;
+  constexpr bool SUM_SMEM = HD == 64 || TILES == 1;
   extern __shared__ __align__(1024) uint8_t smem_pt[];
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem_pt + L::BAR_OFF);
   uint64_t *kv_full = bars, *kv_empty = bars + PT_RING, *s_full = bars + 2 * PT_RING, *p_full = s_full + 2, *q_full = p_full + 2, *drained = q_full + 1,
@@ -132,18 +176,18 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
   volatile uint32_t &s_abort = *(tmem_slot + 1), &s_bad = *(tmem_slot + 2);  // s_bad: zeros stand for infinities or NaN in V
   float *s_pair = reinterpret_cast<float *>(smem_pt + L::PAIR_OFF);  // [tile][half][row]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t g = blockIdx.y, split = blockIdx.z, rows_total = a.T * a.G, row0 = blockIdx.x * 128u * a.tiles;
-  const uint32_t n_tiles = a.tiles == 2u && rows_total - row0 > 128u ? 2u : 1u;
+  const uint32_t g = blockIdx.y, split = blockIdx.z, rows_total = a.T * a.G, row0 = blockIdx.x * 128u * TILES;
+  const uint32_t n_tiles = TILES == 2 && rows_total - row0 > 128u ? 2u : 1u;
 
   if (threadIdx.x == 0) {
     s_abort = 0u, s_bad = 0u;
     for (int i = 0; i < PT_RING; i++) mbar_init(&kv_full[i], 1u), mbar_init(&kv_empty[i], 1u);
-    for (int t = 0; t < 2; t++) mbar_init(&s_full[t], 1u), mbar_init(&p_full[t], 8u);
+    for (int t = 0; t < TILES; t++) mbar_init(&s_full[t], 1u), mbar_init(&p_full[t], 8u);
     mbar_init(q_full, 8u * n_tiles), mbar_init(drained, 1u), mbar_init(tail, 1u);
-    for (int i = 0; i < 8; i++) mbar_init(&pair_bar[i], 2u);
+    for (int i = 0; i < 4 * TILES; i++) mbar_init(&pair_bar[i], 2u);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == PT_SOFT_WARPS) {
+  if (warp == SOFT_WARPS) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -154,15 +198,15 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
   pdl_prologue();
 
   // positions of this split: whole blocks of 128, dealt evenly (read by each role where it first needs them: the Q rows do not)
-  uint32_t pos0 = 0u, p_hi = 0u, b0 = 0u, n = 0u;
+  uint32_t pos0 = 0u, first_lim = 0u, p_hi = 0u, b0 = 0u, n = 0u, seg = 1u;  // first_lim, p_hi: the fewest / most that a row of the CTA sees
   uint32_t issued = 0u;  // blocks asked for by the loader
   auto positions = [&] {
-    pos0 = *a.pos, p_hi = pos0 + row_token(min(rows_total, row0 + 128u * a.tiles) - 1u, a.inv_g) + 1u;
+    pos0 = *a.pos, first_lim = pos0 + row_token(row0, a.inv_g) + 1u, p_hi = pos0 + row_token(min(rows_total, row0 + 128u * TILES) - 1u, a.inv_g) + 1u;
     const uint32_t blocks = (p_hi + PT_KEYS - 1u) / PT_KEYS, per = (blocks + gridDim.z - 1u) / gridDim.z;
-    b0 = min(blocks, split * per), n = min(blocks, b0 + per) - b0;
+    b0 = min(blocks, split * per), n = min(blocks, b0 + per) - b0, seg = pt_segment<HD>(blocks, first_lim / PT_KEYS);
   };
 
-  if (warp < PT_SOFT_WARPS) {
+  if (warp < SOFT_WARPS) {
     // ---------------- softmax: eight warps per tile; warp w & 3 of them has 32 rows, one per lane, the two warps of a quarter half the columns each
     const uint32_t t = (uint32_t)warp >> 3, half = ((uint32_t)warp >> 2) & 1u, wq = (uint32_t)warp & 3u, rl = wq * 32u + lane, r = row0 + t * 128u + rl;
     const bool real = r < rows_total;
@@ -218,10 +262,34 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
       }
       positions();
       const uint32_t lim = real ? pos0 + tok + 1u : 0xFFFFFFFFu;  // positions this row sees (rows past the last are never stored)
-      const uint32_t first_lim = pos0 + row_token(row0, a.inv_g) + 1u;  // the fewest that a row of the CTA sees
       float m = -INFINITY, l = 0.0f;  // maximum the row's terms are taken against (log2 units), sum of this thread's terms
+      float m_sum = -INFINITY;        // the maximum that the sums of the segments before are taken against
+      // Those sums, of this thread's half of the row: in shared memory, columns apart by 128 rows, or (two tiles of heads of 128: no
+      // room) where the row itself goes.
+      float *sum_s = reinterpret_cast<float *>(smem_pt + L::SUM_OFF) + (HD == 64 ? t * HD * 128u : 0u) + half * (HD / 2u) * 128u + rl;
+      auto sum_g = [&] {
+        return (a.part ? a.part + (split * (size_t)a.T * a.n_head + (size_t)tok * a.n_head + head) * HD
+                       : reinterpret_cast<float *>(reinterpret_cast<char *>(a.out) + a.out_stride * tok) + (size_t)head * HD) + half * (HD / 2u);
+      };
+      auto add_sums = [&](uint32_t (&v)[32], int c) {  // to columns 32 c .. of the running segment
+        const float f = m_sum == -INFINITY ? 0.0f : ex2(m_sum - m);
+        if (SUM_SMEM) {
+#pragma unroll
+          for (int i = 0; i < 32; i++) v[i] = __float_as_uint(fmaf(sum_s[(32 * c + i) * 128], f, __uint_as_float(v[i])));
+        } else if (real) {
+          const float *row = sum_g() + 32 * c;
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            float x[8];
+            ld8(row + 8 * u, x, a.wide & 4u);
+#pragma unroll
+            for (int e = 0; e < 8; e++) v[8 * u + e] = __float_as_uint(fmaf(x[e], f, __uint_as_float(v[8 * u + e])));
+          }
+        }
+      };
       bool ok = true;
-      for (uint32_t j = 0; j < n; j++) {
+      uint32_t at = 0;  // blocks of the running segment
+      for (uint32_t j = 0; j < n; j++, at++) {
         ok = __all_sync(0xFFFFFFFFu, mbar_wait(&s_full[t], j & 1u, &s_abort));  // the warp goes on or gives up as one
         if (!ok) break;
         tc_fence_after();
@@ -257,6 +325,24 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
         if (lane == 0) mbar_arrive(pair);  // this warp has read all of S: the other may put P into it (waited for below, under the exponentials)
         if (j == 0) {
           m = mx;
+        } else if (at == seg) {  // the segment's O (complete: s_full says so) joins the sums, and O starts anew
+#pragma unroll 1
+          for (int c = 0; c < HD / 64; c++) {
+            uint32_t v[32];
+            tc_ld32(o_col + 32u * c, v);
+            tc_wait_ld();
+            if (j != seg) add_sums(v, c);
+            if (SUM_SMEM) {
+#pragma unroll
+              for (int i = 0; i < 32; i++) sum_s[(32 * c + i) * 128] = __uint_as_float(v[i]);
+            } else if (real) {
+              float *row = sum_g() + 32 * c;
+#pragma unroll
+              for (int u = 0; u < 4; u++) st8(row + 8 * u, v + 8 * u, a.wide & 4u);
+            }
+          }
+          m_sum = m, at = 0;
+          if (mx > m) l = m == -INFINITY ? l : l * ex2(m - mx), m = mx;
         } else {
           const bool grow = mx > m + 8.0f || (m == -INFINITY && mx > m);
           if (__any_sync(0xFFFFFFFFu, grow)) {  // rescale what the row has (PV of the block before has completed: s_full says so)
@@ -361,6 +447,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
           uint32_t v[32];
           tc_ld32(o_col + 32u * c, v);
           tc_wait_ld();
+          if (n > seg) add_sums(v, c);
           if (s_bad && real) {  // what the zeros in V stand for, for the positions that this row sees (every such p is positive)
             const uint32_t k1 = min(lim, (b0 + n) * PT_KEYS);
 #pragma unroll 1
@@ -425,7 +512,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
         }
       }
     }
-  } else if (warp == PT_SOFT_WARPS) {
+  } else if (warp == SOFT_WARPS) {
     // ---------------- MMA issue: one thread ----------------
     positions();
     if (lane == 0 && n > 0u) {
@@ -435,21 +522,20 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
       auto qk = [&](uint32_t t, uint32_t buf) {
         const uint32_t qa = q_base + t * 2u * L::QTERM, kb = kv_base + buf * L::BLOCK;
 #pragma unroll
-        for (uint32_t s = 0; s < HD / 16; s++) {
+        for (uint32_t i = 0; i < HD / 8; i++) {  // the low terms first: see above
+          const uint32_t s = i % (HD / 16), lo = i < HD / 16 ? L::QTERM : 0u;
           const uint64_t b = tc_desc128(kb + (s >> 2) * 16384u + (s & 3u) * 32u, 16u, 1024u);  // 64-column boxes; 8-row groups 1024 bytes apart
-          tc_mma(tmem + t * 128u, tc_desc(qa + s * 4096u, 2048u, 128u), b, id_qk, s ? 1u : 0u);
-          tc_mma(tmem + t * 128u, tc_desc(qa + L::QTERM + s * 4096u, 2048u, 128u), b, id_qk, 1u);
+          tc_mma(tmem + t * 128u, tc_desc(qa + lo + s * 4096u, 2048u, 128u), b, id_qk, i ? 1u : 0u);
         }
         tc_commit(&s_full[t]);
       };
       auto pv = [&](uint32_t t, uint32_t buf, uint32_t acc) {
         const uint32_t vb = kv_base + buf * L::BLOCK;
 #pragma unroll
-        for (uint32_t s = 0; s < PT_KEYS / 16; s++) {  // 16 keys: two groups of 8 rows (1024 bytes apart); 64-column boxes 16 KB apart
+        for (uint32_t i = 0; i < PT_KEYS / 8; i++) {  // 16 keys: two groups of 8 rows (1024 bytes apart); 64-column boxes 16 KB apart
+          const uint32_t s = i % (PT_KEYS / 16), lo = i < PT_KEYS / 16 ? 16u : 0u;
           const uint64_t b = tc_desc128(vb + s * 2048u, 16384u, 1024u);
-          const uint32_t pa = tmem + t * 128u + (s >> 1) * 32u + (s & 1u) * 8u;
-          tc_mma_ta(tmem + 256u + t * HD, pa, b, id_pv, (acc | s) ? 1u : 0u);
-          tc_mma_ta(tmem + 256u + t * HD, pa + 16u, b, id_pv, 1u);
+          tc_mma_ta(tmem + 256u + t * HD, tmem + t * 128u + (s >> 1) * 32u + (s & 1u) * 8u + lo, b, id_pv, (acc | i) ? 1u : 0u);
         }
       };
       // Blocks in ring order K0 V0 K1 V1 ...: number u sits in buffer u % 3. Issue order QK0 QK1 | PV0 QK0' PV1 QK1' | ...:
@@ -463,14 +549,16 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
         for (uint32_t t = 0; t < n_tiles; t++) qk(t, 0u);
         tc_commit(&kv_empty[0]);
       }
-      for (uint32_t j = 0; j < n && ok; j++) {
+      uint32_t at = 0;  // blocks of the running segment
+      for (uint32_t j = 0; j < n && ok; j++, at++) {
+        if (at == seg) at = 0;
         const uint32_t uv = 2u * j + 1u, uk = 2u * j + 2u;
         ok = full(uv) && (j + 1u == n || full(uk));
         for (uint32_t t = 0; t < n_tiles && ok; t++) {
           ok = mbar_wait(&p_full[t], j & 1u, &s_abort);
           if (!ok) break;
           tc_fence_after();
-          pv(t, uv % PT_RING, j);
+          pv(t, uv % PT_RING, at);
           if (t + 1u == n_tiles) tc_commit(&kv_empty[uv % PT_RING]);
           if (j + 1u < n) {
             qk(t, uk % PT_RING);
@@ -515,8 +603,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
   tc_fence_before();
   __syncthreads();
   if (s_abort) {  // (nobody sets it any more) do not leave while MMAs or copies still use this CTA's memory
-    if (warp == PT_SOFT_WARPS && lane == 0) tc_commit(drained), mbar_drain(drained, 0u);
-    if (warp == PT_SOFT_WARPS + 1 && lane == 0) {
+    if (warp == SOFT_WARPS && lane == 0) tc_commit(drained), mbar_drain(drained, 0u);
+    if (warp == SOFT_WARPS + 1 && lane == 0) {
       for (uint32_t u = issued > PT_RING ? issued - PT_RING : 0u; u < issued; u++) {
         const bool ragged = (u & 1u) && p_hi - (b0 + (u >> 1)) * PT_KEYS < PT_KEYS;
         mbar_drain(ragged ? tail : &kv_full[u % PT_RING], ragged ? 0u : (u / PT_RING) & 1u);
@@ -524,8 +612,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
     }
     // The rows say so too (a caller may have given no error word): NaN, in the outputs or in the records that the merge reads.
     const float nan = __int_as_float(0x7FFFFFFF);
-    const uint32_t n_rows = min(rows_total - row0, 128u * a.tiles), nbq = a.n_head * HD / 32u;
-    for (uint32_t i = threadIdx.x; i < n_rows * (HD / 32u); i += PT_THREADS) {
+    const uint32_t n_rows = min(rows_total - row0, 128u * TILES), nbq = a.n_head * HD / 32u;
+    for (uint32_t i = threadIdx.x; i < n_rows * (HD / 32u); i += THREADS) {
       const uint32_t r = row0 + i / (HD / 32u), tok = row_token(r, a.inv_g), head = g * a.G + (r - tok * a.G), b = i % (HD / 32u);
       if (a.part) {
         if (b < 2u) a.ml[(split * (size_t)a.T * a.n_head + (size_t)tok * a.n_head + head) * 2u + b] = nan;
@@ -539,7 +627,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) attn_prefill_tc_kernel(const Pt
     __syncthreads();
   }
   __syncwarp();
-  if (warp == PT_SOFT_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+  if (warp == SOFT_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
 
 // The splits' records of a (token, head) row -> its output and Q8 copy: hd / 4 lanes per row, four floats each. A record (-inf, 0)
@@ -607,14 +695,15 @@ size_t attn_prefill_scratch_bytes(uint32_t n_head, uint32_t hd, uint32_t T) {
   return std::min((size_t)PT_MAX_SPLITS * T * n_head, (size_t)PT_MAX_RECORDS) * (hd + 2u) * sizeof(float) + 256u;
 }
 
-template <int HD>
+template <int HD, int TILES>
 static int launch_pt(const PtArgs &a, const void *kc, const void *vc, uint32_t splits, cudaStream_t st) {
   CUtensorMap km, vm;
   if (int r = tc_map_2d_f16(&km, kc, HD, (uint64_t)a.n_kv * a.kv_len, 64u, PT_KEYS)) return r;
   if (int r = tc_map_2d_f16(&vm, vc, HD, (uint64_t)a.n_kv * a.kv_len, 64u, PT_KEYS)) return r;
-  auto k = attn_prefill_tc_kernel<HD>;
+  auto k = attn_prefill_tc_kernel<HD, TILES>;
   if (int r = ensure_dynamic_smem(reinterpret_cast<const void *>(k), PtSmem<HD>::TOTAL)) return r;
-  IEB_LAUNCH_PDL("attn_prefill_tc_kernel", k, dim3((a.T * a.G + 128u * a.tiles - 1u) / (128u * a.tiles), a.n_kv, splits), dim3(PT_THREADS), PtSmem<HD>::TOTAL, st, a, km, vm);
+  IEB_LAUNCH_PDL("attn_prefill_tc_kernel", k, dim3((a.T * a.G + 128u * TILES - 1u) / (128u * TILES), a.n_kv, splits), dim3((8 * TILES + 2) * 32), PtSmem<HD>::TOTAL,
+                 st, a, km, vm);
   if (splits > 1u)
     IEB_LAUNCH_PDL("attn_prefill_merge_kernel", attn_prefill_merge_kernel<HD>, dim3((a.T * a.n_head + 1024u / HD - 1u) / (1024u / HD)), dim3(256), 0, st,
                    static_cast<const float *>(a.part), static_cast<const float *>(a.ml), splits, a.T, a.n_head, a.out, a.oq, a.out_stride, a.oq_stride, a.wide & 1u);
@@ -643,9 +732,10 @@ int attn_prefill_tc(const float *d_q, const void *d_kc, const void *d_vc, float 
   a.inv_g = 1.0f / (float)a.G;
   // (a caller without scratch has not said how many positions there are: one split, and as many blocks as the chunk itself has)
   pick_shape(T * a.G, n_kv, ((d_scratch ? positions : T) + PT_KEYS - 1u) / PT_KEYS, T * n_head, hd, d_scratch != nullptr, &tiles, &splits);
-  a.tiles = tiles;
   if (splits > 1u) a.part = d_scratch, a.ml = d_scratch + (size_t)splits * T * n_head * hd;
-  return hd == 64 ? launch_pt<64>(a, d_kc, d_vc, splits, st) : launch_pt<128>(a, d_kc, d_vc, splits, st);
+  if (((uintptr_t)(a.part ? a.part : d_out) & 31u) == 0u && (a.part || (out_stride & 31u) == 0u)) a.wide |= 4u;
+  if (hd == 64) return tiles == 1u ? launch_pt<64, 1>(a, d_kc, d_vc, splits, st) : launch_pt<64, 2>(a, d_kc, d_vc, splits, st);
+  return tiles == 1u ? launch_pt<128, 1>(a, d_kc, d_vc, splits, st) : launch_pt<128, 2>(a, d_kc, d_vc, splits, st);
 }
 
 }  // namespace ieb

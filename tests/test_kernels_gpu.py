@@ -763,7 +763,10 @@ def test_attention_prefill_chunk(ora, cuda, n_head, n_kv, hd, T, pos0):
 
 
 @pytest.mark.parametrize("n_head,n_kv,hd,T,pos0", [(8, 2, 128, 64, 0), (8, 2, 128, 70, 58), (40, 8, 128, 256, 1000), (16, 2, 64, 130, 897), (5, 1, 128, 2, 6000),
-                                                   (3, 3, 64, 129, 127), (28, 4, 128, 37, 3)])
+                                                   (3, 3, 64, 129, 127), (28, 4, 128, 37, 3),
+                                                   # many KV heads: one and two tiles, sums of several accumulations in shared memory and in the rows
+                                                   (64, 16, 128, 64, 0), (64, 16, 128, 70, 58), (32, 32, 64, 129, 127), (112, 16, 128, 37, 3), (64, 16, 64, 300, 700),
+                                                   (320, 40, 128, 256, 600)])
 @pytest.mark.parametrize("split", [False, True])
 def test_attention_prefill_tiles(cuda, n_head, n_kv, hd, T, pos0, split):
     """The tcgen05 chunk attention at the edges of its tiles: rows that fill one or two 128-row tiles exactly or spill into the
@@ -793,6 +796,35 @@ def test_attention_prefill_tiles(cuda, n_head, n_kv, hd, T, pos0, split):
     assert torch.isfinite(out).all()
     assert (out.double() - want).abs().max() <= 1e-4 * want.abs().max()
     assert (oq == K.quant_q8(out)).all()
+
+
+@pytest.mark.parametrize("n_head,n_kv,hd,T,pos0,bound", [
+    (64, 16, 128, 256, 8000, 5.5e-6), (32, 32, 64, 256, 8000, 5.5e-6), (64, 16, 128, 256, 1000, 1.2e-6), (64, 16, 64, 256, 256, 6.0e-7),
+    (64, 16, 128, 256, 0, 4.5e-7), (64, 16, 128, 77, 500, 8.5e-7), (40, 8, 128, 256, 4000, 3.0e-6)])
+@pytest.mark.parametrize("split", [False, True])
+def test_attention_prefill_error_against_64_bits(cuda, n_head, n_kv, hd, T, pos0, bound, split):
+    """The chunk attention's error (2-norm, against a 64-bit softmax over the same cache) is no larger than that of a kernel which
+    accumulates a quarter of the positions at a time with mma.sync (4.5e-7, 7.3e-7, 1.1e-6, 2.8e-6 and 5.2e-6 at 0, 256, 1000, 4000 and
+    8000 positions for heads of 128; 5.3e-7 at 256 and 5.0e-6 at 8000 for heads of 64: the bounds are 5 to 10 % above). The tensor cores cut off
+    what an accumulation loses, 2^-25.7 of it per MMA: all positions of 8000 in one accumulation, high and low terms in turn, give 2.0e-5."""
+    import torch
+
+    from amd_c_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(pos0 + T)
+    n, G = pos0 + T, n_head // n_kv
+    kc, vc = (torch.randn((n_kv, n, hd), generator=gen, device=cuda).half() for _ in range(2))
+    q = torch.randn((T, n_head * hd), generator=gen, device=cuda)
+    pos = torch.tensor([pos0], dtype=torch.int32, device=cuda)
+    out = K.attn_prefill_split(q, kc, vc, pos, n_head, n_kv, hd, n)[0] if split else K.attn_prefill(q, kc, vc, pos, n_head, n_kv, hd)[0]
+    mask = torch.arange(n, device=cuda)[None, :] > (pos0 + torch.arange(T, device=cuda))[:, None]
+    diff = norm = 0.0
+    for g in range(n_kv):
+        s = torch.einsum("tgd,nd->tgn", q.double().view(T, n_kv, G, hd)[:, g], kc[g].double()) / hd ** 0.5
+        want = torch.softmax(s.masked_fill(mask[:, None, :], float("-inf")), 2) @ vc[g].double()
+        diff += float(((out.double().view(T, n_kv, G, hd)[:, g] - want) ** 2).sum())
+        norm += float((want ** 2).sum())
+    assert (diff / norm) ** 0.5 <= bound, (diff / norm) ** 0.5
 
 
 @pytest.mark.parametrize("n_head,n_kv,hd,T,pos0", [(28, 4, 128, 64, 1000), (8, 1, 64, 96, 1000)])
@@ -835,7 +867,8 @@ def test_attention_prefill_empty_splits(cuda, lib, n_head, n_kv, hd, T, pos0):
     assert int(err.item()) == 0
 
 
-@pytest.mark.parametrize("n_head,n_kv,hd,T,pos0", [(8, 8, 64, 256, 100), (28, 4, 128, 64, 1000), (8, 2, 128, 70, 58), (3, 1, 64, 17, 0)])
+@pytest.mark.parametrize("n_head,n_kv,hd,T,pos0", [(8, 8, 64, 256, 100), (28, 4, 128, 64, 1000), (8, 2, 128, 70, 58), (3, 1, 64, 17, 0),
+                                                   (32, 32, 64, 256, 100), (112, 16, 128, 64, 1000), (64, 16, 128, 70, 58)])
 @pytest.mark.parametrize("split", [False, True])
 def test_attention_prefill_infinite_values(cuda, n_head, n_kv, hd, T, pos0, split):
     """A V value that overflowed the half cache (or a NaN) belongs to the tokens that see its position: the rows of the tokens
