@@ -674,21 +674,30 @@ static int tc_map_2d_f16(CUtensorMap *map, const void *base, uint64_t cols, uint
 }
 
 // Tiles per CTA and splits of the positions. A CTA occupies an SM, so the CTAs run in whole waves of the SM count; the time of
-// a choice in microseconds: waves x (blocks per split x what a block takes + start and end of a CTA), plus, with splits, the
-// merge launch and the partial rows' way through memory. Two tiles hide each other's softmax (3.5 us a block of 128 positions
-// for 256 rows, against 2.9 for 128 alone), one tile spreads a short chunk over more SMs and has half the rows to load and store.
-static void pick_shape(uint32_t rows, uint32_t n_kv, uint32_t blocks, uint32_t all_rows, uint32_t hd, bool may_split, uint32_t *tiles, uint32_t *splits) {
-  const uint32_t sms = (uint32_t)sm_count();
+// a choice in microseconds: waves x (blocks per split x what a block takes + start and end of a CTA + accumulations that join the
+// rows' sums), plus, with splits, the merge launch and the partial rows' way through memory. Two tiles hide each other's softmax,
+// one tile spreads a short chunk over more SMs and has half the rows to load and store. The figures are fitted to 2 .. 256
+// tokens, 2 .. 8 KV heads of 2 .. 7 query heads at 0 .. 16000 positions with one to sixteen splits (900 timings, 6 % off on
+// average; the choice made by them 1 % behind the best one): us per block, per CTA, less per CTA of few rows, per accumulation.
+struct PtTime {
+  float block, cta, few_rows, sum;
+};
+static float pick_shape(uint32_t rows, uint32_t n_kv, uint32_t blocks, uint32_t all_rows, uint32_t hd, bool may_split, uint32_t *tiles, uint32_t *splits) {
+  static const PtTime time[2][2] = {{{2.12f, 5.4f, 1.24f, 0.56f}, {2.4f, 8.7f, 0.0f, 1.1f}}, {{2.52f, 7.8f, 2.5f, 0.75f}, {2.95f, 13.0f, 0.0f, 6.5f}}};  // [head size][tiles]
+  const uint32_t sms = (uint32_t)sm_count(), seg = hd == 64 ? pt_segment<64>(blocks, 0u) : pt_segment<128>(blocks, 0u);
   float best = 1e30f;
   for (uint32_t t = 1; t <= 2u; t++) {
+    const PtTime &c = time[hd == 64 ? 0 : 1][t - 1u];
     const uint32_t ctas = (rows + 128u * t - 1u) / (128u * t) * n_kv;
+    const float cta = c.cta - c.few_rows * (rows < 128u ? 1.0f - (float)rows / 128.0f : 0.0f);
     for (uint32_t s = 1; s <= (may_split ? PT_MAX_SPLITS : 1u) && s <= blocks && (s == 1u || s * all_rows <= PT_MAX_RECORDS); s++) {
-      const uint32_t per = (blocks + s - 1u) / s, waves = (ctas * s + sms - 1u) / sms;
-      float cost = (float)waves * (t == 2u ? (float)per * 3.5f + 8.0f : (float)per * 2.9f + 5.0f);
-      if (s > 1u) cost += 3.5f + (float)s * (float)all_rows * (float)hd * 8.0f / 4.0e6f;
+      const uint32_t per = (blocks + s - 1u) / s, waves = (ctas * s + sms - 1u) / sms, joins = (per + seg - 1u) / seg - 1u;
+      float cost = (float)waves * ((float)per * c.block + cta + (float)joins * c.sum);
+      if (s > 1u) cost += 2.3f + (float)s * (float)all_rows * (float)hd * 8.0f / 10.8e6f;
       if (cost < best) best = cost, *tiles = t, *splits = s;
     }
   }
+  return best;
 }
 
 size_t attn_prefill_scratch_bytes(uint32_t n_head, uint32_t hd, uint32_t T) {
