@@ -10,7 +10,7 @@
 // Bound: the tensor pipe (4 x 128 x 128 x hd multiply-adds per block and tile, about 2000 cycles at hd 128); the softmax of
 // one tile (some 900 issue slots per warp) runs under the MMAs of the other. The kernel it replaced (mma.sync, 16 rows per
 // CTA: the cache re-read from L2 for every 16 rows, 84 TFLOP/s) took 2048 us for 256 tokens x 40 heads at 32.5 k positions
-// and 192 us for 256 x 28 at 4 k.
+// and 192 us for 256 x 28 at 4 k. It is kept for small chunks (attn_decode.cu; the rule is at attn_prefill_tc).
 //
 // Tensor memory (512 columns): S / P of the two tiles (128 each; 32 keys' S columns become 16 columns of p_hi and 16 of p_lo
 // in place, so a thread never holds more than 32 scores), O of the two tiles (hd each).
@@ -137,10 +137,6 @@ __device__ __forceinline__ void store_row4(float *out, size_t out_stride, uint8_
 }
 
 __device__ __forceinline__ __half2 as_half2(uint32_t w) { return *reinterpret_cast<const __half2 *>(&w); }
-// Two halves in a word: all ones in the place of each that is an infinity or a NaN.
-__device__ __forceinline__ uint32_t half_bad(uint32_t w) {
-  return ((w & 0x7C00u) == 0x7C00u ? 0xFFFFu : 0u) | ((w & 0x7C000000u) == 0x7C000000u ? 0xFFFF0000u : 0u);
-}
 
 // r / G for r below 2^22 (exact: r + 0.5 is at least 0.5 / G away from a multiple of G, the product's error below 2^-23 of it)
 __device__ __forceinline__ uint32_t row_token(uint32_t r, float inv_g) { return (uint32_t)(((float)r + 0.5f) * inv_g); }
@@ -700,6 +696,16 @@ static float pick_shape(uint32_t rows, uint32_t n_kv, uint32_t blocks, uint32_t 
   return best;
 }
 
+// Microseconds of the mma.sync form, fitted the same way (1100 timings at up to 16000 positions, 5 % off on average): its CTAs are
+// up to 16 rows each, so there are many; a walk in tiles of 64 positions slows down with the CTAs that read the cache at once, and
+// above what the SMs hold together comes in waves (heads of 128) or shares the SMs further (heads of 64).
+static float mma_time(uint32_t ctas, uint32_t positions, uint32_t hd) {
+  const float sms = (float)sm_count(), n = (float)ctas, busy = std::min(n, sms);
+  const float tile = (hd == 64 ? 0.57f : 0.94f) + 0.0036f * std::max(0.0f, busy - 32.0f);
+  const float waves = hd == 64 ? std::max(1.0f, n / 300.0f) : ceilf(n / (2.0f * sms));
+  return (hd == 64 ? 3.0f : 5.0f) + 2.0f * busy / sms + (float)((positions + 63u) / 64u) * tile * waves;
+}
+
 size_t attn_prefill_scratch_bytes(uint32_t n_head, uint32_t hd, uint32_t T) {
   return std::min((size_t)PT_MAX_SPLITS * T * n_head, (size_t)PT_MAX_RECORDS) * (hd + 2u) * sizeof(float) + 256u;
 }
@@ -739,8 +745,13 @@ int attn_prefill_tc(const float *d_q, const void *d_kc, const void *d_vc, float 
   uint32_t splits = 1u, tiles = 1u;
   a.wide = ((((uintptr_t)d_out | out_stride) & 15u) == 0u ? 1u : 0u) | ((((uintptr_t)d_q | q_stride) & 15u) == 0u ? 2u : 0u);
   a.inv_g = 1.0f / (float)a.G;
-  // (a caller without scratch has not said how many positions there are: one split, and as many blocks as the chunk itself has)
-  pick_shape(T * a.G, n_kv, ((d_scratch ? positions : T) + PT_KEYS - 1u) / PT_KEYS, T * n_head, hd, d_scratch != nullptr, &tiles, &splits);
+  // Where the start and end of this kernel's CTAs, or one walk over many positions by few of them, take longer than the mma.sync form
+  // does, that one runs (48 tokens of 28 x 4 heads of 128 at position 100: 9.5 against 13.5 us; 2 at 0: 5.8 / 7.8; 16 at 16000 without
+  // scratch 240 / 310). A caller who has not said how many positions there are: while it has an SM per CTA.
+  const uint32_t mma_ctas = (T + 16u / a.G - 1u) / (16u / a.G) * n_kv;
+  const float tc_time = pick_shape(T * a.G, n_kv, (std::max(positions, T) + PT_KEYS - 1u) / PT_KEYS, T * n_head, hd, d_scratch != nullptr, &tiles, &splits);
+  if (positions ? mma_time(mma_ctas, positions, hd) <= tc_time : mma_ctas <= (uint32_t)sm_count())
+    return attn_prefill_mma(d_q, d_kc, d_vc, d_out, d_oq, d_pos, n_head, n_kv, hd, kv_len, T, q_stride, out_stride, oq_stride, st);
   if (splits > 1u) a.part = d_scratch, a.ml = d_scratch + (size_t)splits * T * n_head * hd;
   if (((uintptr_t)(a.part ? a.part : d_out) & 31u) == 0u && (a.part || (out_stride & 31u) == 0u)) a.wide |= 4u;
   if (hd == 64) return tiles == 1u ? launch_pt<64, 1>(a, d_kc, d_vc, splits, st) : launch_pt<64, 2>(a, d_kc, d_vc, splits, st);

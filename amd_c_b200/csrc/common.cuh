@@ -124,6 +124,10 @@ __device__ __forceinline__ float ld_stream_f32(const void *p) {
   return v;
 }
 
+// Two halves in a word: all ones in the place of each that is an infinity or a NaN.
+__device__ __forceinline__ uint32_t half_bad(uint32_t w) {
+  return ((w & 0x7C00u) == 0x7C00u ? 0xFFFFu : 0u) | ((w & 0x7C000000u) == 0x7C000000u ? 0xFFFF0000u : 0u);
+}
 __device__ __forceinline__ float h2f(uint16_t h) { return __half2float(__ushort_as_half(h)); }
 
 // dot4 of four unsigned bytes with four signed bytes, added to c (dp4a.u32.s32).

@@ -233,16 +233,17 @@ int ie_b200_attn_persistent(const float *d_qkv, void *d_kc, void *d_vc, const fl
 /* Causal attention of a prompt chunk: T tokens at positions *d_pos .. *d_pos + T - 1 whose (rotated) K / V rows are
  * already in the half-precision cache (ie_b200_rope_kv); token t sees positions 0 .. *d_pos + t. The role of
  * ie_attn_pfg / ie_attn_fa (kernels/ie_kernels.c:3471-3693; dispatch src/hip.c:1432-1463): the
- * (token, query head) rows of one KV head share passes over the cache on the tcgen05 tensor cores (f16 MMA, fp32 softmax and
- * accumulation, q and p carried as two f16 terms). hd 64 or 128; d_q rows of n_head * hd floats (already rotated), output rows and their
- * Q8 copies (d_oq may be NULL) as ie_b200_attn_decode; strides in bytes. No scratch. */
+ * (token, query head) rows of one KV head share passes over the cache on the tensor cores, small chunks by mma.sync, others by
+ * tcgen05 (f16 MMA, fp32 softmax and accumulation, q and p carried as two f16 terms). hd 64 or 128; d_q rows of n_head * hd floats (already rotated), output rows and their
+ * Q8 copies (d_oq may be NULL) as ie_b200_attn_decode; strides in bytes. No scratch. Rows are NaN where a bounded
+ * wait inside the kernel ran out. */
 int ie_b200_attn_prefill(const float *d_q, const void *d_kc, const void *d_vc, float *d_out, void *d_oq, const uint32_t *d_pos,
                          uint32_t n_head, uint32_t n_kv, uint32_t hd, uint32_t kv_len, uint32_t T, size_t q_stride, size_t out_stride,
                          size_t oq_stride, void *stream);
 
 /* The same with the positions split over several CTAs per row tile and the partial rows merged by a second kernel: what a
  * chunk of few rows far into the context needs to fill the GPU (the engine's form). positions: *d_pos + T as the host knows it
- * (it sizes the grid; the result does not depend on it). d_scratch: ie_b200_attn_prefill_scratch_bytes() bytes, 16-byte
+ * (it sizes the grid; the result depends on it in the order of the sums only). d_scratch: ie_b200_attn_prefill_scratch_bytes() bytes, 16-byte
  * aligned; d_err (may be NULL): set to 5 if a bounded wait inside the kernel ran out. */
 size_t ie_b200_attn_prefill_scratch_bytes(uint32_t n_head, uint32_t hd, uint32_t T);
 int ie_b200_attn_prefill_split(const float *d_q, const void *d_kc, const void *d_vc, float *d_out, void *d_oq, const uint32_t *d_pos,
