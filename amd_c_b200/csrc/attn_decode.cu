@@ -936,12 +936,22 @@ __global__ void __launch_bounds__(AM_THREADS, 2) attn_prefill_mma_kernel(const P
     __syncthreads();
     issue(it + NB - 1u);
     if (tile_lo + TILE > pos0 + 1u) {  // the first token does not see all of this tile
+      uint4 *p = reinterpret_cast<uint4 *>(reinterpret_cast<char *>(vbuf + buf * TILE_ELEMS) + (size_t)my_row * ROW * 2u + my_piece);
+      __half2 top = __float2half2_rn(0.0f);
 #pragma unroll
       for (int j = 0; j < TILE / RPP; j++) {
-        uint4 *p = reinterpret_cast<uint4 *>(reinterpret_cast<char *>(vbuf + buf * TILE_ELEMS) + (size_t)(my_row + RPP * j) * ROW * 2u + my_piece);
-        const uint4 x = *p;
-        const uint4 bad = make_uint4(half_bad(x.x), half_bad(x.y), half_bad(x.z), half_bad(x.w));
-        if (bad.x | bad.y | bad.z | bad.w) *p = make_uint4(x.x & ~bad.x, x.y & ~bad.y, x.z & ~bad.z, x.w & ~bad.w), s_bad = 1u;
+        const uint4 x = p[j * RPP * ROW / 8];
+        top = __hmax2_nan(__hmax2_nan(top, __habs2(as_half2(x.x))), __habs2(as_half2(x.y)));
+        top = __hmax2_nan(__hmax2_nan(top, __habs2(as_half2(x.z))), __habs2(as_half2(x.w)));
+      }
+      if (half_bad(*reinterpret_cast<const uint32_t *>(&top))) {
+#pragma unroll 1
+        for (int j = 0; j < TILE / RPP; j++) {
+          uint4 x = p[j * RPP * ROW / 8];
+          x.x &= ~half_bad(x.x), x.y &= ~half_bad(x.y), x.z &= ~half_bad(x.z), x.w &= ~half_bad(x.w);
+          p[j * RPP * ROW / 8] = x;
+        }
+        s_bad = 1u;
       }
       __syncthreads();
     }
@@ -1008,26 +1018,35 @@ __global__ void __launch_bounds__(AM_THREADS, 2) attn_prefill_mma_kernel(const P
     if (tq == 0) ml[(warp * 16 + r) * 2] = run_m[h], ml[(warp * 16 + r) * 2 + 1] = run_l[h];
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < ROWS * HD; e += AM_THREADS) {
+  for (int e = threadIdx.x; e < (int)nt * G * HD; e += AM_THREADS) {
     const int r = e / HD;
     float M = -INFINITY;
 #pragma unroll
     for (int w = 0; w < AM_WARPS; w++) M = fmaxf(M, ml[(w * 16 + r) * 2]);
-    float L = 0.0f, acc = 0.0f;
+    float L = ml[r * 2 + 1], acc = 0.0f;  // (no maximum: the scores are all NaN, as this sum then is)
+    if (M != -INFINITY) {
+      L = 0.0f;
 #pragma unroll
-    for (int w = 0; w < AM_WARPS; w++) {
-      const float wk = M == -INFINITY ? 1.0f : expf(ml[(w * 16 + r) * 2] - M);  // (all of them: nothing seen, or only NaN)
-      L = fmaf(wk, ml[(w * 16 + r) * 2 + 1], L);
-      acc = fmaf(wk, red[(w * 16 + r) * HD + (e % HD)], acc);
-    }
-    if (s_bad && (uint32_t)(r / G) < nt)
-      for (uint32_t p = (pos0 + 1u) / TILE * TILE; p < pos0 + r / G + 1u; p++) {
-        const float x = __half2float(vh[(size_t)p * HD + e % HD]);
-        if (!(fabsf(x) <= 65504.0f)) acc += x;
+      for (int w = 0; w < AM_WARPS; w++) {
+        const float wk = expf(ml[(w * 16 + r) * 2] - M);
+        L = fmaf(wk, ml[(w * 16 + r) * 2 + 1], L);
+        acc = fmaf(wk, red[(w * 16 + r) * HD + (e % HD)], acc);
       }
-    fin[e] = L != 0.0f ? acc * (1.0f / L) : 0.0f;
+    }
+    fin[e] = acc * (1.0f / L);
   }
   __syncthreads();
+  if (s_bad) {  // what the zeros in V stand for, for the positions that each row sees
+#pragma unroll 1
+    for (int e = threadIdx.x; e < (int)nt * G * HD; e += AM_THREADS) {
+#pragma unroll 1
+      for (uint32_t p = (pos0 + 1u) / TILE * TILE; p < pos0 + e / (G * HD) + 1u; p++) {
+        const float x = __half2float(vh[(size_t)p * HD + e % HD]);
+        if (!(fabsf(x) <= 65504.0f)) fin[e] += x;
+      }
+    }
+    __syncthreads();
+  }
   // ---- write out: one warp per 32 values of a (token, head) row, which is also a Q8 block of that token's output
   const uint32_t nbq = a.n_head * HD / 32u;
   for (int b = warp; b < ROWS * HD / 32; b += AM_WARPS) {

@@ -136,7 +136,6 @@ __device__ __forceinline__ void store_row4(float *out, size_t out_stride, uint8_
   if ((at & 31u) == 0u) reinterpret_cast<float *>(qrow + 32u * (size_t)nbq)[at / 32u] = d, reinterpret_cast<int *>(qrow + 36u * (size_t)nbq)[at / 32u] = sum;
 }
 
-__device__ __forceinline__ __half2 as_half2(uint32_t w) { return *reinterpret_cast<const __half2 *>(&w); }
 
 // r / G for r below 2^22 (exact: r + 0.5 is at least 0.5 / G away from a multiple of G, the product's error below 2^-23 of it)
 __device__ __forceinline__ uint32_t row_token(uint32_t r, float inv_g) { return (uint32_t)(((float)r + 0.5f) * inv_g); }
@@ -689,7 +688,7 @@ static float pick_shape(uint32_t rows, uint32_t n_kv, uint32_t blocks, uint32_t 
     for (uint32_t s = 1; s <= (may_split ? PT_MAX_SPLITS : 1u) && s <= blocks && (s == 1u || s * all_rows <= PT_MAX_RECORDS); s++) {
       const uint32_t per = (blocks + s - 1u) / s, waves = (ctas * s + sms - 1u) / sms, joins = (per + seg - 1u) / seg - 1u;
       float cost = (float)waves * ((float)per * c.block + cta + (float)joins * c.sum);
-      if (s > 1u) cost += 2.3f + (float)s * (float)all_rows * (float)hd * 8.0f / 10.8e6f;
+      if (s > 1u) cost += 2.3f + (float)s * (float)all_rows * (float)hd * 8.0f / 8.5e6f;
       if (cost < best) best = cost, *tiles = t, *splits = s;
     }
   }
@@ -747,10 +746,11 @@ int attn_prefill_tc(const float *d_q, const void *d_kc, const void *d_vc, float 
   a.inv_g = 1.0f / (float)a.G;
   // Where the start and end of this kernel's CTAs, or one walk over many positions by few of them, take longer than the mma.sync form
   // does, that one runs (48 tokens of 28 x 4 heads of 128 at position 100: 9.5 against 13.5 us; 2 at 0: 5.8 / 7.8; 16 at 16000 without
-  // scratch 240 / 310). A caller who has not said how many positions there are: while it has an SM per CTA.
-  const uint32_t mma_ctas = (T + 16u / a.G - 1u) / (16u / a.G) * n_kv;
+  // scratch 240 / 310). A caller who has not said how many positions there are: while its CTAs fill one wave (two per SM), where the
+  // cache may be long one per SM (77 tokens of 32 x 8 heads of 128, 160 CTAs: 9.6 / 10.5 us at 0, 51 / 50 at 2000, 347 / 313 at 16000).
+  const uint32_t mma_ctas = (T + 16u / a.G - 1u) / (16u / a.G) * n_kv, sms = (uint32_t)sm_count();
   const float tc_time = pick_shape(T * a.G, n_kv, (std::max(positions, T) + PT_KEYS - 1u) / PT_KEYS, T * n_head, hd, d_scratch != nullptr, &tiles, &splits);
-  if (positions ? mma_time(mma_ctas, positions, hd) <= tc_time : mma_ctas <= (uint32_t)sm_count())
+  if (positions ? mma_time(mma_ctas, positions, hd) <= tc_time : mma_ctas <= (kv_len <= 4096u ? 2u : 1u) * sms)
     return attn_prefill_mma(d_q, d_kc, d_vc, d_out, d_oq, d_pos, n_head, n_kv, hd, kv_len, T, q_stride, out_stride, oq_stride, st);
   if (splits > 1u) a.part = d_scratch, a.ml = d_scratch + (size_t)splits * T * n_head * hd;
   if (((uintptr_t)(a.part ? a.part : d_out) & 31u) == 0u && (a.part || (out_stride & 31u) == 0u)) a.wide |= 4u;

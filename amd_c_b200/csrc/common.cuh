@@ -124,6 +124,7 @@ __device__ __forceinline__ float ld_stream_f32(const void *p) {
   return v;
 }
 
+__device__ __forceinline__ __half2 as_half2(uint32_t w) { return *reinterpret_cast<const __half2 *>(&w); }
 // Two halves in a word: all ones in the place of each that is an infinity or a NaN.
 __device__ __forceinline__ uint32_t half_bad(uint32_t w) {
   return ((w & 0x7C00u) == 0x7C00u ? 0xFFFFu : 0u) | ((w & 0x7C000000u) == 0x7C000000u ? 0xFFFF0000u : 0u);
