@@ -22,7 +22,7 @@
 // weights and the tokens' 128 bytes each of activations per 32-column stage, as many stages as fit.
 // Matrices with few rows (3584 x 18944: 14 CTAs) are split along K over grid.z, every split writing its partial sums to
 // scratch, which a second kernel adds in split order (deterministic). Every mbarrier wait is bounded by wall time and reports through the device
-// error word; a warp goes on or gives up as one, and a CTA that gave up waits for its copies and MMAs on their way before it
+// error word; a warp goes on as one, waiting or not, and a CTA that gave up waits for its copies and MMAs on their way before it
 // frees its tensor memory and ends.
 //
 // Half precision has a narrow exponent range, so both sides are scaled by exact powers of two before they are split (a value
@@ -265,9 +265,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
   // its way before the wait for the activations
   const uint32_t t_p = (uint32_t)warp >> 3, row0 = m0 + t_p * 128u + ((uint32_t)warp & 7u) * 16u;
   uint8_t *raw = sR + (uint32_t)warp * 2u * RS_BYTES<KIND>;
-  const uint32_t kq = kb0 & ~3u;  // raw stages start at multiples of four blocks; a split may start inside one
-  if (warp < TC_PROD_WARPS) {
-    if (n_it > 0u) rs_issue<KIND>(a.w, a.rowb, a.rows, a.nb, rs_smem(raw), row0, kq, lane);
+  if (warp < TC_PROD_WARPS) {  // (raw stages start at multiples of four blocks; a split may start inside one)
+    if (n_it > 0u) rs_issue<KIND>(a.w, a.rowb, a.rows, a.nb, rs_smem(raw + ((kb0 >> 2) & 1u) * RS_BYTES<KIND>), row0, kb0 & ~3u, lane);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   pdl_wait();  // the expanded activations (and the residual) are complete
@@ -281,18 +280,19 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
     const uint32_t r = lane & 15u, hf = (uint32_t)lane >> 4, rl = ((uint32_t)warp & 7u) * 16u + r;  // row of the raw stage, column half, row in the tile
     const uint32_t dst0 = t_p * 2 * TC_A_TILE + (rl >> 3) * 128u + (rl & 7u) * 16u + hf * 2u * 2048u;
     uint32_t s = 0, par = 1u;  // the first round finds every stage empty
-    for (uint32_t it = 0; it < n_it; it++) {
-      const uint32_t b = kb0 + it, i = b & 3u, q = (b - kq) >> 2;  // block, its place in raw stage q
-      const uint8_t *src = raw + (q & 1u) * RS_BYTES<KIND>;
-      if (i == 0u || it == 0u) {  // the next four blocks have arrived; ask for the four after them, whose place all lanes have done with
+    for (uint32_t b = kb0; b < kb1; b++) {
+      const uint32_t i = b & 3u;  // its place in the raw stage, which lies in place (b / 4) mod 2
+      const uint8_t *src = raw + ((b >> 2) & 1u) * RS_BYTES<KIND>;
+      if (i == 0u || b == kb0) {  // the next four blocks have arrived; ask for the four after them, whose place all lanes have done with
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncwarp();
-        if (kq + 4u * q + 4u < kb1) rs_issue<KIND>(a.w, a.rowb, a.rows, a.nb, rs_smem(raw + ((q + 1u) & 1u) * RS_BYTES<KIND>), row0, kq + 4u * q + 4u, lane);
+        const uint32_t next = (b | 3u) + 1u;
+        if (next < kb1) rs_issue<KIND>(a.w, a.rowb, a.rows, a.nb, rs_smem(raw + ((next >> 2) & 1u) * RS_BYTES<KIND>), row0, next, lane);
         asm volatile("cp.async.commit_group;" ::: "memory");
       }
       uint32_t hi[8], lo[8];
       tc_convert<KIND>(src, r, i, b, hf, a.w_scale, hi, lo);
-      if (!__all_sync(0xFFFFFFFFu, mbar_wait(&empty_a[s], par, &s_abort))) break;  // the warp goes on or gives up as one
+      mbar_wait(&empty_a[s], par, &s_abort);  // (after giving up the lanes go on together, without waiting: nobody stores the results)
       uint8_t *dst = sA + s * TC_A_STAGE + dst0;
 #pragma unroll
       for (int c = 0; c < 2; c++) {  // 8-column chunks 2 hf + c of the block
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
       if (++s == a.sa) s = 0u, par ^= 1u;
     }
     // ---------------- epilogue: accumulators -> token rows ----------------
-    const bool finished = __all_sync(0xFFFFFFFFu, mbar_wait(done, 0u, &s_abort));
+    const bool finished = __all_sync(0xFFFFFFFFu, mbar_wait(done, 0u, &s_abort) && !s_abort);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (finished) {
       // warp w reads lanes 32 (w & 3) .. + 31 of tensor memory (a warp reaches the quarter w mod 4 only): tile (w >> 2) & 1,
