@@ -153,10 +153,11 @@ __global__ void __launch_bounds__(256) swiglu_il_kernel(const float *gu, float *
 }
 
 // The same for whole blocks and 16-byte aligned rows: four outputs per thread, eight threads per block (two 16-byte loads, one
-// store and three exchanges instead of five; the bound for a chunk is the pass over memory: 256 x 18944, 27 us with one output per thread).
+// store and three exchanges instead of five; the bound for a chunk is the pass over memory: 256 x 18944, 24 us with one output per
+// thread, 10 with four). A thread's four quotients and exponentials are a longer chain, though: see ie_b200_swiglu_il.
 __global__ void __launch_bounds__(256) swiglu_il4_kernel(const float *gu, float *h, uint32_t n, uint8_t *q, size_t gs, size_t hs, size_t qs) {
   pdl_prologue();
-  const uint32_t t = blockIdx.y, i = 4u * (blockIdx.x * 256u + threadIdx.x);
+  const uint32_t t = blockIdx.y, i = 4u * (blockIdx.x * blockDim.x + threadIdx.x);
   const bool ok = i < n;
   float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
   if (ok) {
@@ -465,8 +466,14 @@ extern "C" int ie_b200_swiglu_il(const float *d_gu, float *d_h, uint32_t n, void
   if (((uintptr_t)d_gu & 7u) || (gu_stride & 7u)) return fail(IE_B200_E_ARG, "ie_b200_swiglu_il: the gate / up pairs must be 8-byte aligned");
   if (n == 0 || T == 0) return IE_B200_OK;
   if (T > 65535u) return fail(IE_B200_E_SIZE, "ie_b200_swiglu_il: T %u > 65535", T);
-  if (n % 32u == 0 && !(((uintptr_t)d_gu | gu_stride | (uintptr_t)d_h | h_stride) & 15u) && !(((uintptr_t)d_q | q_stride) & 3u)) {
-    IEB_LAUNCH_PDL("swiglu_il4_kernel", swiglu_il4_kernel, dim3((n / 4u + 255u) / 256u, T), dim3(256), 0, static_cast<cudaStream_t>(stream), d_gu, d_h, n,
+  // Few outputs (a decode step, a few tokens): the shorter chain of one output per thread counts (14336 x 1 1.40 against 1.56 us, x 2
+  // 1.41 / 1.57; level at 8192 x 4). Then four per thread, in small CTAs while those of 256 threads would fill one and a half SM rounds
+  // (14336 x 8 2.16 us with one per thread, 1.64 with 64 threads, 1.77 with 256; x 16 2.29 / 2.35 / 2.64; x 48 4.27 / 3.10 / 3.27; x 64
+  // 5.38 / 4.05 / 3.25).
+  const size_t all = (size_t)n * T;
+  if (all >= 32768u && n % 32u == 0 && !(((uintptr_t)d_gu | gu_stride | (uintptr_t)d_h | h_stride) & 15u) && !(((uintptr_t)d_q | q_stride) & 3u)) {
+    const uint32_t threads = all < 393216u ? 64u : 256u;
+    IEB_LAUNCH_PDL("swiglu_il4_kernel", swiglu_il4_kernel, dim3((n / 4u + threads - 1u) / threads, T), dim3(threads), 0, static_cast<cudaStream_t>(stream), d_gu, d_h, n,
                    static_cast<uint8_t *>(d_q), gu_stride, h_stride, q_stride);
     return IE_B200_OK;
   }

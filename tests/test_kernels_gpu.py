@@ -1151,10 +1151,11 @@ def test_swiglu_inside_the_gemvs(ora, cuda, lib, typ, ffn, dim):
     assert (bits(y.cpu().numpy()) == bits(ora.gemv(kd, dw, ds, dim, ffn, want_q, res=res))).all()
 
 
-@pytest.mark.parametrize("n,T", [(32, 1), (1056, 3), (14336, 1), (18944, 7)])
+@pytest.mark.parametrize("n,T", [(32, 1), (1056, 3), (14336, 1), (18944, 7), (32, 1024), (1056, 32), (1056, 373), (18944, 24)])
 def test_swiglu_interleaved_wide_and_narrow(cuda, lib, n, T):
-    """The four-outputs-per-thread form (rows of whole blocks, 16-byte aligned) against the one-output form, which a result 4
-    bytes off the alignment takes: the same bits, values and Q8 copies, blocks of zeros and infinities among them."""
+    """The four-outputs-per-thread form (rows of whole blocks, 16-byte aligned, 32768 outputs and more: CTAs of 64 threads, from
+    393216 of 256) against the one-output form, which a result 4 bytes off the alignment takes: the same bits, values and Q8
+    copies, blocks of zeros and infinities among them."""
     import torch
 
     from amd_c_b200 import kernels as K
