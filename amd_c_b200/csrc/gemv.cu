@@ -38,16 +38,13 @@ __device__ __forceinline__ void stage_q8(const uint8_t *xq, uint32_t nb, uint4 *
 template <int KIND, int R, int U>
 __global__ void __launch_bounds__(GEMV_THREADS)
 gemv_q_kernel(const uint8_t *__restrict__ w, size_t rowb, uint32_t rows, uint32_t nb, const uint8_t *__restrict__ x, float *y,
-              const float *__restrict__ bias, const float *res, size_t xs, size_t ys, size_t rs) {
+              const float *__restrict__ bias, const float *res) {
   extern __shared__ uint4 smem[];
   uint4 *A0 = smem, *A1 = smem + nb;
   float *da = reinterpret_cast<float *>(smem + 2u * nb);
   int *as = reinterpret_cast<int *>(da + nb);
-  const uint32_t t = blockIdx.y;
-  stage_q8(x + t * xs, nb, A0, A1, da, as);
+  stage_q8(x, nb, A0, A1, da, as);
   __syncthreads();
-  y = reinterpret_cast<float *>(reinterpret_cast<char *>(y) + t * ys);
-  if (res) res = reinterpret_cast<const float *>(reinterpret_cast<const char *>(res) + t * rs);
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t stride = gridDim.x * GEMV_WARPS * R;
@@ -180,9 +177,8 @@ static int launch_q(const void *w, uint32_t rows, uint32_t cols, const void *x, 
   const size_t smem = (size_t)nb * 40u;
   auto k = gemv_q_kernel<KIND, R, U>;
   if (int r = ensure_dynamic_smem(reinterpret_cast<const void *>(k), smem)) return r;
-  const dim3 grid(gemv_grid(rows, GEMV_WARPS * R, 8), T);
-  k<<<grid, GEMV_THREADS, smem, st>>>(static_cast<const uint8_t *>(w), row_bytes_of(KIND, cols), rows, nb, static_cast<const uint8_t *>(x), y,
-                                      bias, res, xs, ys, rs);
+  k<<<gemv_grid(rows, GEMV_WARPS * R, 8), GEMV_THREADS, smem, st>>>(static_cast<const uint8_t *>(w), row_bytes_of(KIND, cols), rows, nb,
+                                                                    static_cast<const uint8_t *>(x), y, bias, res);
   IEB_LAUNCHED("gemv_q_kernel");
   return IE_B200_OK;
 }
