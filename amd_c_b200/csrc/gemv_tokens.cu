@@ -8,6 +8,8 @@
 // Measured, dp4a -> now, 6 tokens: 28672 x 4096 Q4_0 58 -> 22 us, 4096 x 14336 Q4_0 49 -> 16, 128256 x 4096 Q4_0 222 -> 81, 37888 x
 // 3584 Q4_K 86 -> 29, 3584 x 18944 Q6_K 88 -> 28; 2 tokens: 41 -> 21, 35 -> 14, 155 -> 80, 55 -> 28, 58 -> 26; 16 tokens: 154 -> 35,
 // 101 -> 30, 646 -> 126, 197 -> 42, 185 -> 50.
+// Rows whose activations do not fit (see gemv_tokens_phases) are worked in phases: Q8_0 28672 x 4096 6 / 16 tokens 68 -> 23 / 111 -> 61 us, 5120 x
+// 17408 86 -> 32 / 179 -> 63.
 //
 // Order: the one-token GEMV gives lane l of a warp the blocks l, l + 32, ... in order and adds the 32 lane sums by a tree
 // (16, 8, 4, 2, 1). Warp w of the eight that share a 16-row tile keeps the sums of "lanes" 4 w .. 4 w + 3 in registers (four
