@@ -798,6 +798,38 @@ def test_attention_prefill_tiles(cuda, n_head, n_kv, hd, T, pos0, split):
     assert (oq == K.quant_q8(out)).all()
 
 
+@pytest.mark.parametrize("n_head,n_kv,hd,T,pos0", [(320, 40, 128, 256, 600), (64, 16, 128, 70, 500), (64, 16, 64, 70, 500), (8, 2, 128, 20, 30), (40, 8, 64, 6, 3000)])
+@pytest.mark.parametrize("split", [False, True])
+def test_attention_prefill_rows_off_their_alignment(cuda, lib, n_head, n_kv, hd, T, pos0, split):
+    """Query rows on 8-byte and output rows on 4-byte boundaries (what the entries take) give the aligned rows' bits: both kernels, one
+    and two tiles, sums of several accumulations in shared memory and in the output rows."""
+    import torch
+
+    from amd_c_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(n_head + T)
+    n, w = pos0 + T, n_head * hd
+    kc, vc = (torch.randn((n_kv, n, hd), generator=gen, device=cuda).half() for _ in range(2))
+    q = torch.randn((T, w), generator=gen, device=cuda)
+    pos = torch.tensor([pos0], dtype=torch.int32, device=cuda)
+    scratch = torch.empty(lib.ie_b200_attn_prefill_scratch_bytes(n_head, hd, T), dtype=torch.uint8, device=cuda)
+    q_flat, out_flat = torch.zeros(T * (w + 2) + 2, device=cuda), torch.zeros(T * (w + 3) + 1, device=cuda)
+    q_flat[2:].view(T, w + 2)[:, :w] = q
+    out = torch.empty((T, w), device=cuda)
+
+    def run(qp, qs, op, os_):
+        st = torch.cuda.current_stream().cuda_stream
+        args = (qp, kc.data_ptr(), vc.data_ptr(), op, None, pos.data_ptr(), n_head, n_kv, hd, n, T, qs, os_, 0)
+        K.check(lib.ie_b200_attn_prefill_split(*args, n, scratch.data_ptr(), None, st) if split else lib.ie_b200_attn_prefill(*args, st))
+
+    run(q.data_ptr(), 4 * w, out.data_ptr(), 4 * w)
+    run(q_flat.data_ptr() + 8, 4 * (w + 2), out_flat.data_ptr() + 4, 4 * (w + 3))
+    got = out_flat[1:].view(T, w + 3)
+    assert torch.isfinite(out).all()
+    assert torch.equal(got[:, :w].view(torch.int32), out.view(torch.int32))
+    assert (got[:, w:] == 0).all() and float(out_flat[0]) == 0.0  # nothing beside the rows
+
+
 @pytest.mark.parametrize("n_head,n_kv,hd,T,pos0,bound", [
     (64, 16, 128, 256, 8000, 5.5e-6), (32, 32, 64, 256, 8000, 5.5e-6), (64, 16, 128, 256, 1000, 1.2e-6), (64, 16, 64, 256, 256, 6.0e-7),
     (64, 16, 128, 256, 0, 4.5e-7), (64, 16, 128, 77, 500, 8.5e-7), (40, 8, 128, 256, 4000, 3.0e-6)])
