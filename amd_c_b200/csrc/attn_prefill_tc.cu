@@ -2,7 +2,7 @@
 // T tokens at positions *pos .. *pos + T - 1 whose K / V rows are already in the half-precision cache; the role of
 // ie_attn_pfg / ie_attn_fa (kernels/ie_kernels.c:3471-3693; dispatch src/hip.c:1432-1463).
 //
-// The rows of one KV head are its (token, query head) pairs, token-major: T x G of them. A CTA takes 256 rows (two tiles of
+// The rows of one KV head are its (token, query head) pairs, token-major: T x G of them. A CTA takes 128 or 256 rows (tiles of
 // 128 = the rows of one MMA) of one KV head and one split of the positions, and walks the split's cache rows in blocks of
 // 128: S = Q K^T into tensor memory, softmax by one thread per row, P back into the columns of S, O += P V. Q and P are
 // carried as two f16 terms (22 significant bits, as everywhere on the half cache), K and V are exact, sums are fp32:
@@ -65,24 +65,6 @@ __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
-}
-
-// Two floats in a register pair: one packed instruction for two of them.
-__device__ __forceinline__ uint64_t f32x2(float x, float y) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-  return r;
-}
-__device__ __forceinline__ void f32x2_parts(uint64_t r, float &x, float &y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(r)); }
-__device__ __forceinline__ uint64_t f32x2_fma(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ uint64_t f32x2_add(uint64_t a, uint64_t b) {
-  uint64_t r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
 }
 
 // Eight neighbouring floats of a row: one 32-byte access (whole sectors, however far apart the lanes' rows lie) where aligned.
@@ -356,7 +338,8 @@ __global__ void __launch_bounds__((8 * TILES + 2) * 32, 1) attn_prefill_tc_kerne
           }
         }
         const float nm = m == -INFINITY ? 0.0f : -m;
-        uint64_t sc2 = f32x2(a.scale_log2, a.scale_log2), nm2 = f32x2(nm, nm), sum2 = f32x2(0.0f, 0.0f);
+        const f32x2 sc2 = pk2(a.scale_log2, a.scale_log2), nm2 = pk2(nm, nm);
+        f32x2 sum2 = pk2(0.0f, 0.0f);
 #pragma unroll
         for (int c = 0; c < 2; c++) {
           uint32_t v[32], p[32];
@@ -364,13 +347,13 @@ __global__ void __launch_bounds__((8 * TILES + 2) * 32, 1) attn_prefill_tc_kerne
 #pragma unroll
           for (int i = 0; i < 16; i++) {
             float x, y;
-            f32x2_parts(f32x2_fma(f32x2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), sc2, nm2), x, y);
+            unpk2(fma2(pk2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), sc2, nm2), x, y);
             x = ex2(x), y = ex2(y);
-            const uint64_t xy = f32x2(x, y);
-            sum2 = f32x2_add(sum2, xy);
+            const f32x2 xy = pk2(x, y);
+            sum2 = add2(sum2, xy);
             const __half2 h = __floats2half2_rn(x, y);
             const float2 hf = __half22float2(h);
-            f32x2_parts(f32x2_add(xy, f32x2(-hf.x, -hf.y)), x, y);
+            unpk2(add2(xy, pk2(-hf.x, -hf.y)), x, y);
             const __half2 lo = __floats2half2_rn(x, y);
             p[i] = *reinterpret_cast<const uint32_t *>(&h), p[16 + i] = *reinterpret_cast<const uint32_t *>(&lo);
           }
@@ -382,7 +365,7 @@ __global__ void __launch_bounds__((8 * TILES + 2) * 32, 1) attn_prefill_tc_kerne
         }
         {
           float x, y;
-          f32x2_parts(sum2, x, y);
+          unpk2(sum2, x, y);
           l += x + y;
         }
         if (t == 0u && k0 + PT_KEYS > first_lim) {  // the first tile's warps, ahead of every product with this block of V

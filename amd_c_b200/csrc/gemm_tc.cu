@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
   const uint32_t t_p = (uint32_t)warp >> 3, row0 = m0 + t_p * 128u + ((uint32_t)warp & 7u) * 16u;
   uint8_t *raw = sR + (uint32_t)warp * 2u * RS_BYTES<KIND>;
   if (warp < TC_PROD_WARPS) {  // (raw stages start at multiples of four blocks; a split may start inside one)
-    if (n_it > 0u) rs_issue<KIND>(a.w, a.rowb, a.rows, a.nb, rs_smem(raw + ((kb0 >> 2) & 1u) * RS_BYTES<KIND>), row0, kb0 & ~3u, lane);
+    if (n_it > 0u) rs_issue<KIND>(a.w, a.rowb, a.rows, a.nb, smem_u32(raw + ((kb0 >> 2) & 1u) * RS_BYTES<KIND>), row0, kb0 & ~3u, lane);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   pdl_wait();  // the expanded activations (and the residual) are complete
@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncwarp();
         const uint32_t next = (b | 3u) + 1u;
-        if (next < kb1) rs_issue<KIND>(a.w, a.rowb, a.rows, a.nb, rs_smem(raw + ((next >> 2) & 1u) * RS_BYTES<KIND>), row0, next, lane);
+        if (next < kb1) rs_issue<KIND>(a.w, a.rowb, a.rows, a.nb, smem_u32(raw + ((next >> 2) & 1u) * RS_BYTES<KIND>), row0, next, lane);
         asm volatile("cp.async.commit_group;" ::: "memory");
       }
       uint32_t hi[8], lo[8];

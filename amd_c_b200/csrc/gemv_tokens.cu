@@ -108,7 +108,7 @@ __device__ __forceinline__ void gt_stage_act(const GtArgs &a, uint32_t t0, uint3
 // The four blocks of a stage: acc[i][h][n] += block 4 w + i, rows g + 8 h, tokens 2 t and 2 t + 1 of token tile n.
 template <int KIND, int NT>
 __device__ __forceinline__ void gt_step(const uint8_t *stp, uint32_t b0, const uint8_t *sB, const uint8_t *sD, f32x2 (&acc)[4][2][NT], int lane) {
-  const uint32_t st = rs_smem(stp), g = (uint32_t)lane >> 2, t = lane & 3u;
+  const uint32_t st = smem_u32(stp), g = (uint32_t)lane >> 2, t = lane & 3u;
   const uint32_t lr = lane & 15u;                      // ldmatrix: lanes 0..15 give the rows of the first pair of matrices,
   const uint32_t lh = (uint32_t)lane >> 4;             // lanes 16..31 those of the second
   float s0[2], s1[2];                                  // K kinds: thread t works out the scales of block t for rows g, g + 8
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemv_tokens_kernel(const GtArgs
   auto issue = [&]() {
     if (in < items) {
       if (it_j == 0u) rr.set(a.w, a.rowb, a.rows, nb, it_tile * 16u, lane);
-      rs_issue_rows<KIND>(rr, nb, rs_smem(ring + it_stage * STAGE), 32u * it_j + 4u * w, lane);
+      rs_issue_rows<KIND>(rr, nb, smem_u32(ring + it_stage * STAGE), 32u * it_j + 4u * w, lane);
       in++;
       if (++it_j == steps) it_j = 0, it_tile += stride;
     }

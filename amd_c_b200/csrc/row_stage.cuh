@@ -1,6 +1,6 @@
 // row_stage.cuh -- a warp's private stage of raw weights in shared memory: 16 rows x 4 blocks of a row panel, brought by
-// cp.async with whole 64- or 128-byte runs of a row per request (one row per lane would touch 32 lines with every request),
-// and pairs of floats worked by one instruction. Shared by the multi-token GEMV and the prompt-chunk GEMM.
+// cp.async with whole 64- or 128-byte runs of a row per request (one row per lane would touch 32 lines with every request).
+// Shared by the multi-token GEMV and the prompt-chunk GEMM.
 #pragma once
 
 #include "common.cuh"
@@ -13,31 +13,6 @@ namespace ieb {
 template <int KIND>
 constexpr uint32_t RS_BYTES = KIND == IE_B200_MAT_Q4 ? 1152u : KIND == IE_B200_MAT_Q8 ? 2176u : KIND == IE_B200_MAT_Q4K ? 1280u : 1728u;
 
-// two floats in a register pair, every operation rounded to nearest on its own
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pk2(float lo, float hi) {
-  f32x2 v;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-  return v;
-}
-__device__ __forceinline__ void unpk2(f32x2 v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-
-__device__ __forceinline__ uint32_t rs_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 // N bytes into shared memory, asynchronously: the first `most` of them from global memory (none if !ok), the rest zeros
 template <int N>
 __device__ __forceinline__ void rs_cp(uint32_t dst, const void *src, bool ok, uint32_t most = N) {

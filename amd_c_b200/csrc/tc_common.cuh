@@ -11,7 +11,6 @@ namespace ieb {
 
 constexpr uint64_t TC_WAIT_NS = 2000000000ull;
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ uint64_t tc_now() {
   uint64_t t;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
